@@ -780,6 +780,8 @@ __global__ void __launch_bounds__(engine::kBlockThreads)
         a.ctrl = c;
         a.trace = nullptr;
         a.trace_cap = 0;
+        a.pull_chunks = sp.pull_chunks;
+        a.pull_chunk_cap = sp.pull_chunk_cap;
         a.p = p;
         a.p.total_workload0 = (long long)bq.csr.nedges;
         BCApp app = bq.app;
@@ -925,7 +927,14 @@ sg_status prepare_batch(sg_ctx *ctx, sgb::Workspace &ws, std::vector<engine::Bat
     // chunks are cut on the 4-edge grid: at most one more per heavy vertex than deg / chunk_edges rounded up
     const uint32_t chunk_cap = (uint32_t)(ne_max / p.chunk_edges + 2ull * heavy_cap + 2);
     TB *buf, *tmp;
-    uint32_t *qq, *bm, *fl, *mid, *chunk, *counter;
+    uint32_t *qq, *bm, *fl, *mid, *chunk, *counter, *tiles = nullptr;
+    uint4 *pchunks = nullptr;
+    // pull rounds (hybrid policy or a forced pull) with load balancing: min-relax
+    // functors take edge tiles, the others chunks of their split destinations
+    const bool pulls = (p.forced < 0 || is_pull(p.forced)) && p.lb_pull != LB_NONE;
+    constexpr bool kTiles = has_min_relax<App, TB, TW>::value;
+    const size_t n_tiles = pulls && kTiles ? (ne_max + kPullTileEdges - 1) / kPullTileEdges + 1 : 0;
+    const size_t n_pchunks = pulls && !kTiles ? pull_chunk_bound(ne_max) : 0;
     HeavyItem<TB> *heavy;
     Ctrl *ctrl;
     const size_t T = n_teams;
@@ -939,6 +948,8 @@ sg_status prepare_batch(sg_ctx *ctx, sgb::Workspace &ws, std::vector<engine::Bat
     // two heavy-vertex tables per team (one per round parity)
     if ((st = ws_get(ctx, ws, "b_heavy", T * 2 * heavy_cap, &heavy)) != SG_OK) return st;
     if ((st = ws_get(ctx, ws, "b_chunk", T * 2 * chunk_cap, &chunk)) != SG_OK) return st;
+    if (n_tiles && (st = ws_get(ctx, ws, "b_tiles", T * n_tiles, &tiles)) != SG_OK) return st;
+    if (n_pchunks && (st = ws_get(ctx, ws, "b_pchunks", T * n_pchunks, &pchunks)) != SG_OK) return st;
     if ((st = ws_get(ctx, ws, "b_ctrl", T, &ctrl)) != SG_OK) return st;
     if ((st = ws_get(ctx, ws, "b_counter", 1, &counter)) != SG_OK) return st;
     // heavy/chunk tables start zeroed so that a stale chunk never names an out-of-range item
@@ -966,6 +977,9 @@ sg_status prepare_batch(sg_ctx *ctx, sgb::Workspace &ws, std::vector<engine::Bat
         s.heavy_cap = heavy_cap;
         s.chunk_cap = chunk_cap;
         s.trace_cap = 0;
+        s.tile_row = tiles ? tiles + t * n_tiles : nullptr;
+        s.pull_chunks = pchunks ? pchunks + t * n_pchunks : nullptr;
+        s.pull_chunk_cap = (uint32_t)n_pchunks;
     }
     // BC: levels, path counts, dependencies, level stack and chunk table per team
     if constexpr (kBC) {

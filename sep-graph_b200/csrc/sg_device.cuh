@@ -233,6 +233,9 @@ __device__ __forceinline__ void bitmap_clear(uint32_t *bm, uint32_t v) { atomicA
 __device__ __forceinline__ void bitmap_set_nr(uint32_t *bm, uint32_t v) {
     asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" ::"l"(bm + (v >> 5)), "r"(1u << (v & 31u)) : "memory");
 }
+__device__ __forceinline__ void bitmap_or_nr(uint32_t *word, uint32_t bits) {
+    asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" ::"l"(word), "r"(bits) : "memory");
+}
 __device__ __forceinline__ void red_add(uint32_t *p, uint32_t v) {
     asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }

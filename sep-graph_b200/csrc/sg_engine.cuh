@@ -89,11 +89,14 @@ struct Counters {
     uint32_t qcount[4];
     uint32_t heavy_enq[4];
     unsigned long long scout[4];
+    // engine pull rounds: 1 when the combine phase left some vertex unscheduled
+    // (multi-source BFS: entries of its touched list)
     uint32_t middle_count, error;
     uint32_t active_count;  // active vertices of a round whose worklist nobody reads (forced TD)
     uint32_t heavy_count[2], chunk_count[2];  // heavy-vertex tables, one set per round parity
     unsigned long long edges_processed;
     uint32_t popped;  // worklist items taken from a bitmap worklist this round
+    uint32_t pull_chunk_count;  // entries of KArgs::pull_chunks in the current pull round
 };
 
 struct Ctrl {
@@ -166,7 +169,7 @@ struct KArgs {
     uint32_t *bitmap[2];
     uint32_t *qflag[3];  // queued bitmap of each worklist slot
     uint32_t nwords;
-    uint32_t *middle;
+    uint32_t *middle;  // bitmap of the vertices a pull round scans (ceil(V / 32) words of a V-entry array)
     HeavyItem<TBuffer> *heavy;  // 2 * heavy_cap items: set k starts at heavy + k * heavy_cap
     uint32_t heavy_cap;
     uint32_t *chunk_owner;      // 2 * chunk_cap entries, likewise
@@ -177,12 +180,29 @@ struct KArgs {
     Params p;
     // --wl_sort: one count per block of the team; null = worklists are not sorted
     uint32_t *sort_counts = nullptr;
-    // Edge-tiled topology-driven pull (functors with PullReduce, unweighted):
-    // tile_row[t] = the in-edge row holding CSC edge t * kPullTileEdges
-    // (ceil(E / kPullTileEdges) + 1 entries, the last = V - 1), filled at the
-    // launch's start; null = the destination-per-lane pull is used instead.
+    // Edge-tiled pull (functors with PullReduce, unweighted, topology-driven;
+    // min-relax functors): tile_row[t] = the in-edge row holding CSC edge
+    // t * kPullTileEdges (ceil(E / kPullTileEdges) + 1 entries, the last =
+    // V - 1), filled at the launch's start or in its first pull round; null =
+    // the destination-per-lane pull is used instead.
     uint32_t *tile_row = nullptr;
+    // Pull over destinations: (vertex, first in-edge, in-edges, -) chunks of
+    // the round's vertices above kPullSplit in-edges, listed by its combine
+    // phase; null = a warp scans the whole in-edge list of such a vertex.
+    uint4 *pull_chunks = nullptr;
+    uint32_t pull_chunk_cap = 0;
 };
+
+// In-degree above which a destination's in-edge list is cut into chunks that
+// all warps share, and the chunk's edges.  A warp scans 32 in-edges per
+// dependent trip (about 1 us), so a 20,000-edge hub held up its round for
+// 2 ms and more; 512 bounds a warp's share of one vertex by 16 trips.
+constexpr uint32_t kPullSplit = 512;
+constexpr uint32_t kPullChunk = 256;
+// Chunks of all split vertices: deg / kPullChunk + 1 each, and at most
+// E / kPullSplit of them.
+inline uint64_t pull_chunk_bound(uint64_t ne) { return ne / kPullChunk + ne / kPullSplit + 2; }
+
 
 // In-edges per warp tile of the edge-tiled pull: 8 per lane, two 16-byte loads.
 constexpr uint32_t kPullTileEdges = 256;
@@ -232,16 +252,20 @@ struct LocalQ {
     uint32_t n[2];
     uint32_t out;  // buffer receiving discoveries
 };
+// Outside push rounds the block queue's memory stages the warps' appends.
+constexpr uint32_t kStageItems = 2 * kLocalCap / kWarpsPerBlock;
 
 // Per-thread accumulators flushed once per phase.
 struct Acc {
     unsigned long long scout_hi, scout_lo;
     uint32_t heavy_hi, heavy_lo;
     unsigned long long edges;
+    uint32_t active;
     __device__ void reset() {
         scout_hi = scout_lo = 0;
         heavy_hi = heavy_lo = 0;
         edges = 0;
+        active = 0;
     }
     __device__ __forceinline__ void count(bool hi, uint32_t deg, uint32_t heavy_threshold) {
         const uint32_t h = deg > heavy_threshold;
@@ -459,20 +483,68 @@ struct EngineKernel {
         if (a.p.collect) acc.count(hi, out_degree(a, v), a.p.heavy_threshold);
     }
 
+    // Adds the block's accumulators to the round's counters, one atomic per
+    // block and counter: all blocks update the same few words, and an atomic
+    // per warp (up to 9,472 warps) queued behind one L2 slice at every phase
+    // end.  All threads of the block call, and the next call comes after a
+    // block barrier (every phase ends in a grid barrier).
     static __device__ void flush_acc(const Args &a, Acc &acc, uint32_t q_hi, uint32_t q_lo) {
-        unsigned long long s0 = dev::warp_sum(acc.scout_hi), s1 = dev::warp_sum(acc.scout_lo);
-        uint32_t h0 = dev::warp_sum(acc.heavy_hi), h1 = dev::warp_sum(acc.heavy_lo);
-        unsigned long long ed = dev::warp_sum(acc.edges);
+        __shared__ unsigned long long part[kWarpsPerBlock][6];
+        unsigned long long x[6] = {dev::warp_sum(acc.scout_hi), dev::warp_sum(acc.scout_lo),
+                                   (unsigned long long)dev::warp_sum(acc.heavy_hi),
+                                   (unsigned long long)dev::warp_sum(acc.heavy_lo), dev::warp_sum(acc.edges),
+                                   (unsigned long long)dev::warp_sum(acc.active)};
         if (dev::lane_id() == 0) {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) part[dev::warp_id()][k] = x[k];
+        }
+        __syncthreads();
+        if (threadIdx.x < 6) {
+            const uint32_t k = threadIdx.x;
+            unsigned long long sum = 0;
+#pragma unroll
+            for (int w = 0; w < kWarpsPerBlock; ++w) sum += part[w][k];
             Counters *n = &a.ctrl->cnt;
-            if (s0) atomicAdd(&n->scout[q_hi], s0);
-            if (h0) atomicAdd(&n->heavy_enq[q_hi], h0);
-            if (s1) atomicAdd(&n->scout[q_lo], s1);
-            if (h1) atomicAdd(&n->heavy_enq[q_lo], h1);
-            if (ed) atomicAdd(&n->edges_processed, ed);
+            if (sum) {
+                if (k < 2) atomicAdd(&n->scout[k == 0 ? q_hi : q_lo], sum);
+                else if (k < 4) atomicAdd(&n->heavy_enq[k == 2 ? q_hi : q_lo], (uint32_t)sum);
+                else if (k == 4) atomicAdd(&n->edges_processed, sum);
+                else atomicAdd(&n->active_count, (uint32_t)sum);
+            }
         }
         acc.reset();
     }
+
+    // A warp's worklist appends of a dense phase, collected in shared memory and
+    // moved to the worklist with one reservation per about 200 items: the
+    // counter is a single word, and one returning atomic per 32 vertices (the
+    // 4.6 M found in a pull round of symmetric RMAT-23 took over 100,000) made
+    // it the phase's bound.  All 32 lanes call both members.
+    struct WarpStage {
+        uint32_t *buf;  // kStageItems entries of this warp
+        uint32_t n;     // filled, the same in every lane
+        __device__ __forceinline__ void append(const Args &a, uint32_t slot, bool want, uint32_t item) {
+            const uint32_t m = __ballot_sync(dev::kFullMask, want);
+            if (want) buf[n + __popc(m & dev::lanemask_lt())] = item;
+            n += __popc(m);
+            if (n > kStageItems - 32) flush(a, slot);
+        }
+        __device__ __forceinline__ void flush(const Args &a, uint32_t slot) {
+            __syncwarp();
+            if (n == 0) return;
+            uint32_t base = 0;
+            if (dev::lane_id() == 0) base = atomicAdd(&a.ctrl->cnt.qcount[slot], n);
+            base = __shfl_sync(dev::kFullMask, base, 0);
+            for (uint32_t i = dev::lane_id(); i < n; i += 32) {
+                if (base + i < a.queue_cap)
+                    a.queue[slot][base + i] = buf[i];
+                else
+                    atomicOr(&a.ctrl->cnt.error, dev::kErrCapacity);
+            }
+            __syncwarp();
+            n = 0;
+        }
+    };
 
     // Append dst to the next worklist(s) if `want`: dedupe through the output
     // slot's queued bitmap, route by IsHighPriority when two-level priority is
@@ -1096,13 +1168,18 @@ struct EngineKernel {
         }
     }
 
-    // Worklist items that a round consumes without popping lose their queued bit.
+    // Worklist items that a round consumes without popping lose their queued
+    // bit.  The input slot's queued bitmap holds exactly the worklist's vertices
+    // here (see --wl_sort below), so this is one pass over V / 8 bytes that also
+    // hands the words to the frontier bitmap, instead of two atomics per item.
     static __device__ void release_input_flags(const Args &a, const Snap &s, bool to_bitmap) {
-        const uint32_t *Q = a.queue[s.qin];
-        for (uint32_t i = gthread(); i < s.F; i += nthreads()) {
-            const uint32_t v = dev::ld_l2(Q + i);
-            dev::bitmap_clear(a.qflag[s.qin], v);
-            if (to_bitmap) dev::bitmap_set(a.bitmap[s.bin], v);  // Queue2Bitmap (driver.cuh:119-129)
+        if (s.F == 0) return;
+        uint32_t *bits = a.qflag[s.qin];
+        for (uint32_t w = gthread(); w < a.nwords; w += nthreads()) {
+            const uint32_t x = dev::ld_l2(bits + w);
+            if (x == 0) continue;
+            bits[w] = 0;
+            if (to_bitmap) a.bitmap[s.bin][w] = x;  // Queue2Bitmap (driver.cuh:119-129)
         }
     }
 
@@ -1415,12 +1492,15 @@ struct EngineKernel {
 
     // ---------------------------------------------------------------- pull
     // CombineValueBuffer over every vertex; scheduled vertices form the middle
-    // list (variants/common.cuh:17-84).  `sync` writes the combined buffer to
+    // set (variants/common.cuh:17-84), kept as a bitmap: a warp combines the 32
+    // vertices of one word, so a word costs one plain store where a list cost
+    // an atomic on one counter.  `sync` writes the combined buffer to
     // tmp (SYNC_PULL_*), else back into buffer (ASYNC_PULL_DD, algo_variants.cuh:842-849).
-    static __device__ void combine_all(App &app, const Args &a, bool sync, bool build_middle = true) {
+    // With `split`, scheduled vertices above kPullSplit in-edges list their chunks.
+    static __device__ void combine_all(App &app, const Args &a, bool sync, bool build_middle, bool split) {
         const uint32_t lane = dev::lane_id();
         const uint32_t N = a.csr.nnodes;
-        Counters *n = &a.ctrl->cnt;
+        bool all = true;
         for (uint32_t base = gwarp() * 32; base < N; base += nwarps() * 32) {
             const uint32_t v = base + lane;
             bool want = false;
@@ -1431,29 +1511,63 @@ struct EngineKernel {
                 else
                     a.buffer[v] = pr.first;
                 want = pr.second;
+                if (want && split) list_pull_chunks(a, v);
             }
-            if (build_middle) dev::warp_append(a.middle, &n->middle_count, a.csr.nnodes, want, v, &n->error);
+            if (build_middle) {
+                const uint32_t m = __ballot_sync(dev::kFullMask, want);
+                if (lane == 0) a.middle[base >> 5] = m;
+                all = all && __all_sync(dev::kFullMask, want || v >= N);
+            }
+        }
+        if (build_middle && !all && lane == 0) a.ctrl->cnt.middle_count = 1;  // every writer stores the same value
+    }
+
+    static __device__ __forceinline__ void list_pull_chunks(const Args &a, uint32_t v) {
+        const uint32_t beg = a.csc.begin_edge(v), deg = a.csc.end_edge(v) - beg;
+        if (deg <= kPullSplit) return;
+        Counters *n = &a.ctrl->cnt;
+        const uint32_t nch = (deg + kPullChunk - 1) / kPullChunk;
+        const uint32_t c0 = atomicAdd(&n->pull_chunk_count, nch);
+        for (uint32_t k = 0; k < nch; ++k) {
+            if (c0 + k < a.pull_chunk_cap)
+                a.pull_chunks[c0 + k] = make_uint4(v, beg + k * kPullChunk, min(kPullChunk, deg - k * kPullChunk), 0);
+            else
+                atomicOr(&n->error, dev::kErrChunkCapacity);
         }
     }
 
-    // Pull into one destination, sequentially over its in-edges (early exit on BREAK).
+    // Pull into one destination, sequentially over its in-edges; *brk = whether
+    // a BREAK ended the scan early.
     static __device__ bool pull_serial(App &app, const Args &a, const Snap &s, uint32_t v, uint32_t beg,
-                                       uint32_t deg, bool dd, bool sync, Acc &acc) {
+                                       uint32_t deg, bool dd, bool sync, Acc &acc, bool *broke) {
         const TB *srcbuf = sync ? a.tmp : a.buffer;
         const uint32_t *bin = a.bitmap[s.bin];
         bool hit = false;
         uint32_t e = beg;
-        for (; e < beg + deg; ++e) {
-            const uint32_t u = a.csc.edge_src(e);
-            if (dd && !dev::bitmap_test(bin, u)) continue;
-            const int st = accumulate<App, TB, TW>(app, a.csc_w, u, v, e, a.buffer + v, dev::ld_l2(srcbuf + u));
-            hit |= acc_success(st);
-            if (!acc_continue(st)) {
+        const uint32_t end = beg + deg;
+        bool brk = false;
+        while (e < end && !brk) {  // four sources and frontier bits in flight per step
+            const uint32_t n = min(4u, end - e);
+            uint32_t u[4];
+            bool cand[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) u[j] = a.csc.edge_src(e + min(j, n - 1));
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) cand[j] = j < n && (!dd || dev::bitmap_test_l1(bin, u[j]));
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+                if (brk || j >= n) continue;
+                if (cand[j]) {
+                    const int st = accumulate<App, TB, TW>(app, a.csc_w, u[j], v, e, a.buffer + v,
+                                                           dev::ld_l2(srcbuf + u[j]));
+                    hit |= acc_success(st);
+                    brk = !acc_continue(st);
+                }
                 ++e;
-                break;
             }
         }
         acc.edges += e - beg;
+        *broke = brk;
         return hit;
     }
 
@@ -1534,7 +1648,7 @@ struct EngineKernel {
             if (k < deg) {
                 const uint32_t e = beg + k;
                 const uint32_t u = a.csc.edge_src(e);
-                if (!dd || dev::bitmap_test(bin, u)) {
+                if (!dd || dev::bitmap_test_l1(bin, u)) {
                     const int st = accumulate<App, TB, TW>(app, a.csc_w, u, v, e, a.buffer + v, dev::ld_l2(srcbuf + u));
                     hit |= acc_success(st);
                     brk = !acc_continue(st);
@@ -1547,27 +1661,57 @@ struct EngineKernel {
         return __any_sync(dev::kFullMask, hit);
     }
 
+    // Pull into the middle set: first the chunks of the split destinations,
+    // then a warp takes one word of the set's bitmap at a time, so the frontier
+    // and queued bits of the vertices that succeed are set with one atomic per
+    // word and array.  Every lane scans the first pull_warp_threshold in-edges
+    // of its own vertex, and the whole warp takes the rest of the longer lists,
+    // one vertex after the other: a functor that stops at its first success
+    // (BFS) seldom gets there, where a warp per longer list meant up to 32
+    // lists one after the other.  BFS on symmetric RMAT-23 (8.4 M vertices),
+    // its two pull rounds 753 + 416 -> 324 + 295 us against a middle list
+    // appended and walked vertex by vertex.
     static __device__ void pull_phase(App &app, const Args &a, const Snap &s, WarpLB<TB> &wlb, bool dd, bool sync,
-                                      int lb, Acc &acc) {
+                                      int lb, Acc &acc, uint32_t *stage) {
         const uint32_t lane = dev::lane_id();
-        const uint32_t M = min(dev::ld_l2(&a.ctrl->cnt.middle_count), a.csr.nnodes);
-        const bool natural = (M == a.csr.nnodes);  // every vertex scheduled: keep CSC order
-        Counters *n = &a.ctrl->cnt;
-        for (uint32_t base = gwarp() * 32; base < M; base += nwarps() * 32) {
-            const uint32_t i = base + lane;
-            const bool valid = i < M;
-            uint32_t v = 0, beg = 0, deg = 0;
+        const uint32_t N = a.csr.nnodes;
+        const bool natural = dev::ld_l2(&a.ctrl->cnt.middle_count) == 0;  // every vertex scheduled
+        const bool split = lb != LB_NONE && a.pull_chunks;
+        WarpStage out{stage, 0};
+        const uint32_t C = split ? min(dev::ld_l2(&a.ctrl->cnt.pull_chunk_count), a.pull_chunk_cap) : 0u;
+        for (uint32_t ch = gwarp(); ch < C; ch += nwarps()) {
+            const uint4 c4 = __ldcg(a.pull_chunks + ch);  // the same chunk in every lane
+            bool want = pull_warp(app, a, s, c4.x, c4.y, c4.z, dd, sync, acc) && dd && lane == 0;
+            if (want) {
+                dev::bitmap_set_nr(a.bitmap[s.bout], c4.x);
+                want = dev::bitmap_set(a.qflag[s.qhi], c4.x);
+                if (want) count_enq(a, acc, true, c4.x);
+            }
+            out.append(a, s.qhi, want, c4.x);
+        }
+        for (uint32_t base = gwarp() * 32; base < N; base += nwarps() * 32) {
+            const uint32_t mw = natural ? dev::kFullMask : dev::ld_l2(a.middle + (base >> 5));
+            if (mw == 0) continue;
+            const uint32_t v = base + lane;
+            const bool valid = v < N && ((mw >> lane) & 1u);
+            uint32_t beg = 0, deg = 0;
             if (valid) {
-                v = natural ? i : dev::ld_l2(a.middle + i);
                 beg = a.csc.begin_edge(v);
                 deg = a.csc.end_edge(v) - beg;
+                if (split && deg > kPullSplit) deg = 0;
             }
-            const bool big = valid && lb != LB_NONE && deg > a.p.pull_warp_threshold;
+            bool big = lb != LB_NONE && deg > a.p.pull_warp_threshold;
             bool hit = false;
-            if (dd && lb != LB_NONE && a.p.pull_coop)
-                hit = pull_coop(app, a, s, wlb, v, beg, valid && !big ? deg : 0u, sync, acc);
-            else if (valid && !big)
-                hit = pull_serial(app, a, s, v, beg, deg, dd, sync, acc);
+            if (dd && lb != LB_NONE && a.p.pull_coop) {
+                hit = pull_coop(app, a, s, wlb, v, beg, big ? 0u : deg, sync, acc);
+            } else {
+                const uint32_t own = big ? a.p.pull_warp_threshold : deg;
+                bool broke;
+                hit = pull_serial(app, a, s, v, beg, own, dd, sync, acc, &broke);
+                beg += own;
+                deg -= own;
+                big = big && !broke;
+            }
             uint32_t bigmask = __ballot_sync(dev::kFullMask, big);
             while (bigmask) {
                 const uint32_t j = __ffs(bigmask) - 1;
@@ -1576,18 +1720,146 @@ struct EngineKernel {
                 const uint32_t bj = __shfl_sync(dev::kFullMask, beg, j);
                 const uint32_t dj = __shfl_sync(dev::kFullMask, deg, j);
                 const bool h = pull_warp(app, a, s, vj, bj, dj, dd, sync, acc);
-                if (lane == j) hit = h;
+                if (lane == j) hit |= h;
             }
-            if (dd) {
-                bool want = valid && hit;
-                if (want) {
-                    dev::bitmap_set(a.bitmap[s.bout], v);
-                    want = dev::bitmap_set(a.qflag[s.qhi], v);
+            const uint32_t m = dd ? __ballot_sync(dev::kFullMask, hit) : 0u;
+            if (m) {
+                uint32_t old = 0;
+                if (lane == 0) {
+                    dev::bitmap_or_nr(a.bitmap[s.bout] + (base >> 5), m);
+                    old = atomicOr(a.qflag[s.qhi] + (base >> 5), m);
                 }
-                dev::warp_append(a.queue[s.qhi], &n->qcount[s.qhi], a.queue_cap, want, v, &n->error);
+                old = __shfl_sync(dev::kFullMask, old, 0);
+                const bool want = ((m & ~old) >> lane) & 1u;
+                out.append(a, s.qhi, want, v);
                 if (want) count_enq(a, acc, true, v);
             }
         }
+        out.flush(a, s.qhi);
+    }
+
+    // Pull of a min-relax functor with every vertex scheduled (SSSP's pull
+    // rounds), tiled over the in-edge array like pull_tiles: a warp takes 256
+    // consecutive in-edges, tests their sources' frontier bits (read through
+    // L1), and only for frontier sources reads the weight and the offered
+    // value; the candidates' minimum per destination is formed in shared memory
+    // and compared with the destination once per (row, tile).  A source's value
+    // may be read from L1 while another warp lowers it: the value of the
+    // combine phase is what the round must offer, and a vertex lowered now is
+    // in the next frontier.  Bound by the chain of L2 trips per tile; the
+    // destination-per-thread scan was bound by its longest list: 2.0 ms per
+    // pull round on a 300,007-vertex R-MAT graph (20,000 in-edges at the hub),
+    // with tiles 0.12 ms.
+    static __device__ void pull_tiles_relax(App &app, const Args &a, const Snap &s, WarpLB<TB> &w, bool dd, bool sync,
+                                            Acc &acc, uint32_t *stage) {
+        if constexpr (has_min_relax<App, TB, TW>::value) {
+            const uint32_t lane = dev::lane_id();
+            const uint32_t V = a.csc.nnodes, E = a.csc.nedges;
+            const uint32_t T = (E + kPullTileEdges - 1) / kPullTileEdges;
+            const uint32_t *crow = a.csc.col_start;
+            const uint32_t *srcs = a.csc.edge_source;
+            const bool aligned = (reinterpret_cast<uintptr_t>(srcs) & 15u) == 0;
+            const uint64_t pol = dev::stream_policy();
+            const TB *offers = sync ? a.tmp : a.buffer;
+            const uint32_t *bin = a.bitmap[s.bin];
+            const TB none = std::numeric_limits<TB>::max();
+            WarpStage out{stage, 0};
+            for (uint32_t t = gwarp(); t < T; t += nwarps()) {
+                const uint32_t e0 = t * kPullTileEdges + lane * 8u;
+                if (lane == 0) acc.edges += min(kPullTileEdges, E - t * kPullTileEdges);
+                uint32_t src[8];
+                if (aligned && e0 + 8u <= E) {
+                    const uint4 x = dev::ldg_v4_stream(srcs + e0, pol), y = dev::ldg_v4_stream(srcs + e0 + 4, pol);
+                    src[0] = x.x, src[1] = x.y, src[2] = x.z, src[3] = x.w;
+                    src[4] = y.x, src[5] = y.y, src[6] = y.z, src[7] = y.w;
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) src[j] = e0 + j < E ? dev::ldg_stream(srcs + e0 + j, pol) : 0u;
+                }
+                uint32_t cand = 0;  // edges of this lane whose source is in the frontier
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (e0 + j < E && (!dd || dev::bitmap_test_l1(bin, src[j]))) cand |= 1u << j;
+                if (!__any_sync(dev::kFullMask, cand != 0)) continue;
+                TB offer[8];
+                uint32_t wt[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const bool c = (cand >> j) & 1u;
+                    offer[j] = c ? dev::ld_l1(offers + src[j]) : none;
+                    wt[j] = c && a.csc_w ? dev::ldg_stream(a.csc_w + e0 + j, pol) : 1u;
+                }
+                const uint32_t rlo = __ldg(a.tile_row + t), rhi = __ldg(a.tile_row + t + 1);
+                const bool in_smem = rhi - rlo < kPullTileRows;
+                if (in_smem) {
+                    for (uint32_t k = lane; k <= rhi - rlo; k += 32) w.rowsum[k] = none;
+                    __syncwarp();
+                }
+                auto flush = [&](uint32_t r, TB v) {
+                    if (v == none) return;
+                    if (in_smem) {
+                        atomicMin(&w.rowsum[r - rlo], v);
+                    } else if (v < dev::ld_l2(a.buffer + r)) {
+                        atomicMin(a.buffer + r, v);
+                        if (dd) mark_pulled(a, s, r, acc);
+                    }
+                };
+                if (cand) {
+                    uint32_t r = row_of(crow, rlo, rhi, e0);
+                    uint32_t next = r + 1 < V ? __ldg(crow + r + 1) : E;
+                    TB run = none;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const uint32_t e = e0 + j;
+                        if ((cand >> j) & 1u) {
+                            if (e >= next) {
+                                flush(r, run);
+                                run = none;
+                                r = row_of(crow, r + 1, rhi, e);
+                                next = r + 1 < V ? __ldg(crow + r + 1) : E;
+                            }
+                            const TB x = app.RelaxCandidate(src[j], r, (TW)wt[j], offer[j]);
+                            run = x < run ? x : run;
+                        }
+                    }
+                    flush(r, run);
+                }
+                if (in_smem) {
+                    __syncwarp();
+                    for (uint32_t k0 = 0; k0 <= rhi - rlo; k0 += 32) {
+                        const uint32_t k = k0 + lane, v = rlo + k;
+                        bool want = false;
+                        if (k <= rhi - rlo) {
+                            const TB x = w.rowsum[k];
+                            if (x != none && x < dev::ld_l2(a.buffer + v)) {
+                                atomicMin(a.buffer + v, x);
+                                want = dd;
+                            }
+                        }
+                        if (want) {
+                            dev::bitmap_set_nr(a.bitmap[s.bout], v);
+                            want = dev::bitmap_set(a.qflag[s.qhi], v);
+                            if (want) count_enq(a, acc, true, v);
+                        }
+                        out.append(a, s.qhi, want, v);
+                    }
+                }
+            }
+            out.flush(a, s.qhi);
+        }
+    }
+
+    // A vertex that a pull round improved, marked by one thread: output
+    // frontier bit, queued bit, worklist entry.
+    static __device__ __forceinline__ void mark_pulled(const Args &a, const Snap &s, uint32_t v, Acc &acc) {
+        dev::bitmap_set_nr(a.bitmap[s.bout], v);
+        if (!dev::bitmap_set(a.qflag[s.qhi], v)) return;
+        const uint32_t pos = atomicAdd(&a.ctrl->cnt.qcount[s.qhi], 1u);
+        if (pos < a.queue_cap)
+            a.queue[s.qhi][pos] = v;
+        else
+            atomicOr(&a.ctrl->cnt.error, dev::kErrCapacity);
+        count_enq(a, acc, true, v);
     }
 
     // Topology-driven pull for functors with PullReduce: the warp walks the
@@ -1820,25 +2092,28 @@ struct EngineKernel {
         return a.p.forced == V_SYNC_PULL_TD || a.p.forced == V_ASYNC_PUSH_TD;
     }
 
-    static __device__ void rebuild(App &app, const Args &a, uint32_t slot, Acc &acc) {
+    static __device__ void rebuild(App &app, const Args &a, uint32_t slot, Acc &acc, uint32_t *stage) {
         const uint32_t lane = dev::lane_id();
         const uint32_t N = a.csr.nnodes;
-        Counters *n = &a.ctrl->cnt;
         if (count_only(a)) {
-            uint32_t cnt = 0;
-            for (uint32_t v = gthread(); v < N; v += nthreads()) cnt += app.App::IsActiveNode(v, dev::ld_l2(a.buffer + v));
-            cnt = dev::warp_sum(cnt);
-            if (lane == 0 && cnt) atomicAdd(&n->active_count, cnt);
+            for (uint32_t v = gthread(); v < N; v += nthreads())
+                acc.active += app.App::IsActiveNode(v, dev::ld_l2(a.buffer + v));
             return;
         }
+        WarpStage out{stage, 0};
         for (uint32_t base = gwarp() * 32; base < N; base += nwarps() * 32) {
             const uint32_t v = base + lane;
-            bool act = false;
-            if (v < N) act = app.App::IsActiveNode(v, dev::ld_l2(a.buffer + v));
-            if (act) act = dev::bitmap_set(a.qflag[slot], v);
-            dev::warp_append(a.queue[slot], &n->qcount[slot], a.queue_cap, act, v, &n->error);
-            if (act) count_enq(a, acc, true, v);
+            const bool act = v < N && app.App::IsActiveNode(v, dev::ld_l2(a.buffer + v));
+            const uint32_t m = __ballot_sync(dev::kFullMask, act);
+            if (m == 0) continue;
+            uint32_t old = 0;
+            if (lane == 0) old = atomicOr(a.qflag[slot] + (base >> 5), m);
+            old = __shfl_sync(dev::kFullMask, old, 0);
+            const bool want = ((m & ~old) >> lane) & 1u;
+            out.append(a, slot, want, v);
+            if (want) count_enq(a, acc, true, v);
         }
+        out.flush(a, slot);
     }
 
     // ---------------------------------------------------------------- leader (block 0, thread 0)
@@ -2042,6 +2317,7 @@ struct EngineKernel {
         rs.heavy_expected = a.p.collect ? he[rs.qin] : (rs.F > 0);
         rs.chunks = pend;
         n->middle_count = 0;
+        n->pull_chunk_count = 0;
         n->active_count = 0;
         n->popped = 0;
         // the previous round's deferred set ran at the start of this round; this
@@ -2102,9 +2378,13 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
         a.qflag[1][w] = 0;
         a.qflag[2][w] = 0;
     }
-    if (a.tile_row) K::compute_tile_rows(a);
+    uint32_t *stage = &lq_block.item[0][0] + dev::warp_id() * kStageItems;  // unused while a push round runs
+    constexpr bool reduce = has_pull_reduce<App, TB>::value && std::is_same<TW, graphs::NoWeight>::value;
+    constexpr bool relax = has_min_relax<App, TB, TW>::value;
+    bool tiles_listed = false;  // tile rows of a min-relax functor's pull rounds are filled
+    if (reduce && a.tile_row) K::compute_tile_rows(a);
     if (!grid_sync(c, tmo, nop)) return false;
-    K::rebuild(app, a, 0, acc);
+    K::rebuild(app, a, 0, acc, stage);
     K::flush_acc(a, acc, 0, 2);
     if (!grid_sync(c, tmo, [&] { K::leader_start(a, ps); })) return false;
 
@@ -2171,7 +2451,7 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
                     K::flush_acc(a, acc, s.qhi, s.qlo);
                     if (!grid_sync(c, tmo, nop)) return false;
                 }
-                K::rebuild(app, a, s.qhi, acc);
+                K::rebuild(app, a, s.qhi, acc, stage);
                 K::flush_acc(a, acc, s.qhi, s.qlo);
                 break;
             }
@@ -2181,13 +2461,19 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
                 const bool dd = is_dd(var);
                 const bool sync = is_sync(var);
                 const bool convert = dd && !is_pull_dd(s.last_variant);
-                constexpr bool reduce = has_pull_reduce<App, TB>::value && std::is_same<TW, graphs::NoWeight>::value;
                 K::clear_dirty(a, s);
                 K::release_input_flags(a, s, convert);
                 const bool reduce_td = reduce && !dd && lb_pull != LB_NONE;  // scans every vertex, no middle list
-                K::combine_all(app, a, sync, !reduce_td);
+                const bool tiles = relax && a.tile_row && lb_pull != LB_NONE && !a.p.pull_coop;
+                if (tiles && !tiles_listed) {  // read after the barrier below
+                    K::compute_tile_rows(a);
+                    tiles_listed = true;
+                }
+                K::combine_all(app, a, sync, !reduce_td, !reduce_td && a.pull_chunks && lb_pull != LB_NONE);
                 if (!grid_sync(c, tmo, nop)) return false;
-                if (reduce_td && a.tile_row) {
+                if (tiles && dev::ld_l2(&c->cnt.middle_count) == 0) {
+                    K::pull_tiles_relax(app, a, s, my_lb, dd, sync, acc, stage);
+                } else if (reduce_td && a.tile_row) {
                     K::pull_tiles(app, a, my_lb, acc);
                 } else if (reduce_td) {
                     K::pull_reduce_td(app, a, s, my_lb, acc);
@@ -2195,12 +2481,12 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
                     if (!grid_sync(c, tmo, nop)) return false;
                     K::pull_reduce_chunks(app, a, set, acc);
                 } else {
-                    K::pull_phase(app, a, s, my_lb, dd, sync, lb_pull, acc);
+                    K::pull_phase(app, a, s, my_lb, dd, sync, lb_pull, acc, stage);
                 }
                 K::flush_acc(a, acc, s.qhi, s.qlo);
                 if (!dd) {
                     if (!grid_sync(c, tmo, nop)) return false;
-                    K::rebuild(app, a, s.qhi, acc);
+                    K::rebuild(app, a, s.qhi, acc, stage);
                     K::flush_acc(a, acc, s.qhi, s.qlo);
                 }
                 break;
@@ -2246,6 +2532,9 @@ struct TeamSpace {
     Ctrl *ctrl;
     sg_round_trace *trace;
     uint32_t cap_v, heavy_cap, chunk_cap, trace_cap;
+    uint32_t *tile_row;  // as KArgs::tile_row and pull_chunks (null where the functor does not take them)
+    uint4 *pull_chunks;
+    uint32_t pull_chunk_cap;
 };
 
 // Per-query result record written when the query finishes.
@@ -2322,6 +2611,9 @@ __global__ void __launch_bounds__(kBlockThreads)
         a.ctrl = c;
         a.trace = nullptr;
         a.trace_cap = 0;
+        a.tile_row = sp.tile_row;
+        a.pull_chunks = sp.pull_chunks;
+        a.pull_chunk_cap = sp.pull_chunk_cap;
         a.p = p;
         a.p.total_workload0 = (long long)bq.csr.nedges;
         if (bq.prio_raw) a.p.prio_init_raw = a.p.prio_step_raw = bq.prio_raw;

@@ -515,6 +515,16 @@ sg_status run_engine(sg_graph *g, App app, const EngineConfig &cfg, TV *value, T
         if (g->has_csc && td_pull && cfg.lb_pull != LB_NONE && nv > 0)
             SG_TRY_CUDA(ctx, ws.get("pull_tiles", (ne + kPullTileEdges - 1) / kPullTileEdges + 1, &a.tile_row));
     }
+    // the other pull rounds (hybrid policy or a forced pull variant): edge tiles
+    // for min-relax functors, chunks of the split destinations for the rest
+    if (g->has_csc && cfg.lb_pull != LB_NONE && (cfg.forced < 0 || is_pull(cfg.forced))) {
+        if constexpr (has_min_relax<App, TB, TW>::value) {
+            SG_TRY_CUDA(ctx, ws.get("pull_tiles", (ne + kPullTileEdges - 1) / kPullTileEdges + 1, &a.tile_row));
+        } else {
+            a.pull_chunk_cap = (uint32_t)pull_chunk_bound(ne);
+            SG_TRY_CUDA(ctx, ws.get("pull_chunks", a.pull_chunk_cap, &a.pull_chunks));
+        }
+    }
 
     SG_TRY_CUDA(ctx, cudaMemsetAsync(a.ctrl, 0, sizeof(Ctrl), ctx->stream));
     SG_TRY_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
