@@ -226,9 +226,14 @@ struct PolicyState {
 
 template <typename TBuffer>
 struct WarpLB {
-    uint32_t excl[32];
-    uint32_t beg[32];
-    uint32_t src[32];
+    union {
+        struct {  // an expansion's items: exclusive degree scan, first edges, sources
+            uint32_t excl[32];
+            uint32_t beg[32];
+            uint32_t src[32];
+        };
+        uint32_t rowbeg[kPullTileRows + 1];  // edge-tiled pull: first edges of the tile's rows and of the next one
+    };
     TBuffer pay[32];
     // topology-driven pull: each lane's first and last (possibly shared) segment
     uint32_t partk[2][32];
@@ -1792,21 +1797,27 @@ struct EngineKernel {
                 const uint32_t rlo = __ldg(a.tile_row + t), rhi = __ldg(a.tile_row + t + 1);
                 const bool in_smem = rhi - rlo < kPullTileRows;
                 if (in_smem) {
+                    load_tile_rows(w, crow, rlo, rhi);
                     for (uint32_t k = lane; k <= rhi - rlo; k += 32) w.rowsum[k] = none;
                     __syncwarp();
                 }
-                auto flush = [&](uint32_t r, TB v) {
+                // rows below are relative to rlo
+                auto row_at = [&](uint32_t k, uint32_t e) {
+                    return in_smem ? tile_row_of(w, k, rhi - rlo, e) : row_of(crow, rlo + k, rhi, e) - rlo;
+                };
+                auto row_end = [&](uint32_t k) { return in_smem ? w.rowbeg[k + 1] : __ldg(crow + rlo + k + 1); };
+                auto flush = [&](uint32_t k, TB v) {
                     if (v == none) return;
                     if (in_smem) {
-                        atomicMin(&w.rowsum[r - rlo], v);
-                    } else if (v < dev::ld_l2(a.buffer + r)) {
-                        atomicMin(a.buffer + r, v);
-                        if (dd) mark_pulled(a, s, r, acc);
+                        atomicMin(&w.rowsum[k], v);
+                    } else if (v < dev::ld_l2(a.buffer + rlo + k)) {
+                        atomicMin(a.buffer + rlo + k, v);
+                        if (dd) mark_pulled(a, s, rlo + k, acc);
                     }
                 };
                 if (cand) {
-                    uint32_t r = row_of(crow, rlo, rhi, e0);
-                    uint32_t next = r + 1 < V ? __ldg(crow + r + 1) : E;
+                    uint32_t r = row_at(0, e0);
+                    uint32_t next = row_end(r);
                     TB run = none;
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
@@ -1815,10 +1826,10 @@ struct EngineKernel {
                             if (e >= next) {
                                 flush(r, run);
                                 run = none;
-                                r = row_of(crow, r + 1, rhi, e);
-                                next = r + 1 < V ? __ldg(crow + r + 1) : E;
+                                r = row_at(r + 1, e);
+                                next = row_end(r);
                             }
-                            const TB x = app.RelaxCandidate(src[j], r, (TW)wt[j], offer[j]);
+                            const TB x = app.RelaxCandidate(src[j], rlo + r, (TW)wt[j], offer[j]);
                             run = x < run ? x : run;
                         }
                     }
@@ -1843,6 +1854,7 @@ struct EngineKernel {
                         }
                         out.append(a, s.qhi, want, v);
                     }
+                    __syncwarp();  // rowbeg and rowsum are free for the next tile
                 }
             }
             out.flush(a, s.qhi);
@@ -1964,6 +1976,26 @@ struct EngineKernel {
         return lo;
     }
 
+    // Row starts of a tile's rows [rlo, rhi] (fewer than kPullTileRows) and of
+    // rhi + 1, read together into shared memory: the lanes then search their
+    // rows there, where a search in the row array itself is up to six
+    // dependent L2 loads per lane.
+    static __device__ __forceinline__ void load_tile_rows(WarpLB<TB> &w, const uint32_t *crow, uint32_t rlo,
+                                                          uint32_t rhi) {
+        for (uint32_t k = dev::lane_id(); k <= rhi - rlo + 1; k += 32) w.rowbeg[k] = __ldg(crow + rlo + k);
+    }
+    // Largest k in [lo, hi] with rowbeg[k] <= e.
+    static __device__ __forceinline__ uint32_t tile_row_of(const WarpLB<TB> &w, uint32_t lo, uint32_t hi, uint32_t e) {
+        while (lo < hi) {
+            const uint32_t mid = lo + (hi - lo + 1) / 2;
+            if (w.rowbeg[mid] <= e)
+                lo = mid;
+            else
+                hi = mid - 1;
+        }
+        return lo;
+    }
+
     // tile_row[] of the edge-tiled pull, once per launch (all threads of the team).
     static __device__ void compute_tile_rows(const Args &a) {
         const uint32_t V = a.csc.nnodes, E = a.csc.nedges;
@@ -2004,27 +2036,33 @@ struct EngineKernel {
 #pragma unroll
                     for (int j = 0; j < 8; ++j) s[j] = e0 + j < E ? dev::ldg_stream(srcs + e0 + j, pol) : 0u;
                 }
+                const uint32_t rlo = __ldg(a.tile_row + t), rhi = __ldg(a.tile_row + t + 1);
+                const bool in_smem = rhi - rlo < kPullTileRows;
                 TB g[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) g[j] = e0 + j < E ? dev::ld_l1(vals + s[j]) : idn;
-                const uint32_t rlo = __ldg(a.tile_row + t), rhi = __ldg(a.tile_row + t + 1);
-                const bool in_smem = rhi - rlo < kPullTileRows;
                 if (in_smem) {
+                    load_tile_rows(w, crow, rlo, rhi);
                     for (uint32_t k = lane; k <= rhi - rlo; k += 32) w.rowsum[k] = idn;
                     if (lane == 0) w.touched = 0ull;
                     __syncwarp();
                 }
-                auto flush = [&](uint32_t r, TB v) {
+                // rows below are relative to rlo
+                auto row_at = [&](uint32_t k, uint32_t e) {
+                    return in_smem ? tile_row_of(w, k, rhi - rlo, e) : row_of(crow, rlo + k, rhi, e) - rlo;
+                };
+                auto row_end = [&](uint32_t k) { return in_smem ? w.rowbeg[k + 1] : __ldg(crow + rlo + k + 1); };
+                auto flush = [&](uint32_t k, TB v) {
                     if (in_smem) {
-                        atomicAdd(&w.rowsum[r - rlo], v);  // shared-memory reduction of the tile's rows
-                        atomicOr(&w.touched, 1ull << (r - rlo));
+                        atomicAdd(&w.rowsum[k], v);  // shared-memory reduction of the tile's rows
+                        atomicOr(&w.touched, 1ull << k);
                     } else {
-                        accumulate<App, TB, TW>(app, a.csc_w, r, r, 0, a.buffer + r, v);
+                        accumulate<App, TB, TW>(app, a.csc_w, rlo + k, rlo + k, 0, a.buffer + rlo + k, v);
                     }
                 };
                 if (e0 < E) {
-                    uint32_t r = row_of(crow, rlo, rhi, e0);
-                    uint32_t next = r + 1 < V ? __ldg(crow + r + 1) : E;
+                    uint32_t r = row_at(0, e0);
+                    uint32_t next = row_end(r);
                     TB run = idn;
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
@@ -2033,8 +2071,8 @@ struct EngineKernel {
                             if (e >= next) {
                                 flush(r, run);
                                 run = idn;
-                                r = row_of(crow, r + 1, rhi, e);
-                                next = r + 1 < V ? __ldg(crow + r + 1) : E;
+                                r = row_at(r + 1, e);
+                                next = row_end(r);
                             }
                             run = app.PullReduce(run, g[j]);
                         }
