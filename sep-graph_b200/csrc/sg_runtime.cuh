@@ -131,6 +131,20 @@ struct Workspace {
         *out = (T *)b.p;
         return cudaSuccess;
     }
+    // Releases the buffers whose names start with `prefix`.
+    void drop(const char *prefix) {
+        for (auto it = bufs.begin(); it != bufs.end();) {
+            if (it->first.compare(0, std::strlen(prefix), prefix) == 0) {
+                if (it->second.p) {
+                    if (ordered()) cudaFreeAsync(it->second.p, *stream);
+                    else cudaFree(it->second.p);
+                }
+                it = bufs.erase(it);
+            } else {
+                ++it;
+            }
+        }
+    }
     size_t total_bytes() const {
         size_t s = 0;
         for (auto &kv : bufs) s += kv.second.bytes;
