@@ -197,8 +197,12 @@ struct LevelStack {
     uint32_t max_levels;
     uint32_t *err;
 
+    // one reservation for the lanes that append together (the counter is one word)
     __device__ __forceinline__ void append(uint32_t v) const {
-        const uint32_t p = atomicAdd(count, 1u);
+        const uint32_t m = __activemask(), leader = (uint32_t)__ffs(m) - 1;
+        uint32_t p = 0;
+        if (dev::lane_id() == leader) p = atomicAdd(count, (uint32_t)__popc(m));
+        p = __shfl_sync(m, p, leader) + __popc(m & dev::lanemask_lt());
         if (p < capacity)
             data[p] = v;
         else
@@ -246,20 +250,41 @@ struct BCForward : AppBase<TValue, TBuffer, TWeight> {
         return utils::pair<TBuffer, bool>(buf, schedule);
     }
 
-    __forceinline__ __device__ void add_sigma(index_t dst, index_t src) const {
-        const unsigned long long s = dev::ld_l2(m_sigmas + src);
+    __forceinline__ __device__ void add_sigma(index_t dst, unsigned long long s) const {
         const unsigned long long old = atomicAdd(m_sigmas + dst, s);
         if (old + s < old) atomicOr(m_stack.err, dev::kErrOverflow);
     }
+    // every vertex found in a round raises the depth to the same level: read it first
+    __forceinline__ __device__ void reach_depth(uint32_t level) const {
+        if (dev::ld_l2(m_p_search_depth) < level) atomicMax(m_p_search_depth, level);
+    }
 
+    // Levels only go down, and a destination below the offered level can neither
+    // take it nor count its paths: most edges of a push round end at that read.
     __forceinline__ __device__ int AccumulateBuffer(index_t src, index_t dst, TBuffer *p_buffer,
                                                     TBuffer buffer) override {
+        const TBuffer cur = dev::ld_l2(p_buffer);
+        if (cur < buffer) return this->ACCUMULATE_FAILURE_CONTINUE;
+        return AccumulatePulled(dst, p_buffer, buffer, dev::ld_l2(m_sigmas + src));
+    }
+
+    // Pull in one call per scanned list: the sources of one destination all
+    // offer the next level, so their path counts are summed in registers
+    // (loads in flight together) and added once, instead of one dependent
+    // atomic minimum and addition per frontier in-neighbour.
+    __forceinline__ __device__ unsigned long long PullTerm(index_t src) const { return dev::ld_l2(m_sigmas + src); }
+    __forceinline__ __device__ unsigned long long PullSum(unsigned long long a, unsigned long long b) const {
+        if (a + b < a) atomicOr(m_stack.err, dev::kErrOverflow);
+        return a + b;
+    }
+    __forceinline__ __device__ int AccumulatePulled(index_t dst, TBuffer *p_buffer, TBuffer buffer,
+                                                    unsigned long long paths) {
         const TBuffer prev = atomicMin(p_buffer, buffer);
         if (prev == kInf) {
-            add_sigma(dst, src);
-            atomicMax(m_p_search_depth, buffer);
+            add_sigma(dst, paths);
+            reach_depth(buffer);
         } else if (dev::ld_l2(p_buffer) == buffer) {
-            add_sigma(dst, src);
+            add_sigma(dst, paths);
         }
         return buffer < prev ? this->ACCUMULATE_SUCCESS_CONTINUE : this->ACCUMULATE_FAILURE_CONTINUE;
     }

@@ -356,6 +356,20 @@ struct has_min_relax<App, TB, TW,
                          std::declval<uint32_t>(), std::declval<uint32_t>(), std::declval<TW>(), std::declval<TB>()))>>
     : std::integral_constant<bool, std::is_same<TB, uint32_t>::value> {};
 
+// Optional functor extension (no reference counterpart): a functor whose
+// frontier sources of one data-driven pull round all offer the same value, and
+// whose AccumulateBuffer adds a term of the source and never breaks, declares
+//   __device__ T PullTerm(index_t src) const                 the source's term
+//   __device__ T PullSum(T a, T b) const                     sum of two
+//   __device__ int AccumulatePulled(index_t dst, TBuffer *p_buffer, TBuffer offer, T sum)
+// (T = unsigned long long; BC's path counts) and the engine pulls a scanned
+// list with one AccumulatePulled call.
+template <typename App, typename = void>
+struct has_pull_term : std::false_type {};
+template <typename App>
+struct has_pull_term<App, std::void_t<decltype(std::declval<const App &>().PullTerm(std::declval<uint32_t>()))>>
+    : std::true_type {};
+
 // Edge range of chunk k of a heavy vertex's list [beg, beg + deg): chunks are
 // cut on the 4-edge grid (from beg rounded down to a multiple of 4) so that
 // every chunk starts on a 16-byte boundary of the edge arrays, which lets a
@@ -1551,6 +1565,32 @@ struct EngineKernel {
         uint32_t e = beg;
         const uint32_t end = beg + deg;
         bool brk = false;
+        if constexpr (has_pull_term<App>::value) {
+            if (dd) {
+                unsigned long long sum = 0;
+                uint32_t from = 0xffffffffu;  // a frontier source
+                for (; e < end; e += 4) {
+                    uint32_t u[4];
+                    bool cand[4];
+                    unsigned long long x[4];
+#pragma unroll
+                    for (uint32_t j = 0; j < 4; ++j) u[j] = a.csc.edge_src(min(e + j, end - 1));
+#pragma unroll
+                    for (uint32_t j = 0; j < 4; ++j) cand[j] = e + j < end && dev::bitmap_test_l1(bin, u[j]);
+#pragma unroll
+                    for (uint32_t j = 0; j < 4; ++j) x[j] = cand[j] ? app.PullTerm(u[j]) : 0ull;
+#pragma unroll
+                    for (uint32_t j = 0; j < 4; ++j) {
+                        sum = app.PullSum(sum, x[j]);
+                        if (cand[j]) from = u[j];
+                    }
+                }
+                acc.edges += deg;
+                *broke = false;
+                if (from == 0xffffffffu) return false;
+                return acc_success(app.AccumulatePulled(v, a.buffer + v, dev::ld_l2(srcbuf + from), sum));
+            }
+        }
         while (e < end && !brk) {  // four sources and frontier bits in flight per step
             const uint32_t n = min(4u, end - e);
             uint32_t u[4];
@@ -1647,6 +1687,29 @@ struct EngineKernel {
         const uint32_t *bin = a.bitmap[s.bin];
         bool hit = false;
         uint32_t scanned = 0;
+        if constexpr (has_pull_term<App>::value) {
+            if (dd) {
+                unsigned long long sum = 0;
+                uint32_t from = 0xffffffffu;
+                for (uint32_t k = lane; k < deg; k += 32) {
+                    const uint32_t u = a.csc.edge_src(beg + k);
+                    if (!dev::bitmap_test_l1(bin, u)) continue;
+                    sum = app.PullSum(sum, app.PullTerm(u));
+                    from = u;
+                }
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) {
+                    const unsigned long long y = __shfl_xor_sync(dev::kFullMask, sum, d);
+                    sum = app.PullSum(sum, y);
+                }
+                const uint32_t m = __ballot_sync(dev::kFullMask, from != 0xffffffffu);
+                if (lane == 0) acc.edges += deg;
+                if (m == 0) return false;
+                from = __shfl_sync(dev::kFullMask, from, __ffs(m) - 1);
+                if (lane == 0) hit = acc_success(app.AccumulatePulled(v, a.buffer + v, dev::ld_l2(srcbuf + from), sum));
+                return __any_sync(dev::kFullMask, hit);
+            }
+        }
         for (uint32_t off = 0; off < deg; off += 32) {
             const uint32_t k = off + lane;
             bool brk = false;
