@@ -46,31 +46,6 @@ __global__ void validate_csr_kernel(const uint32_t *row, const uint32_t *col, co
     if (w && dev::lane_id() == 0 && sum != 0) atomicAdd(&chk->weight_sum, sum);
 }
 
-// Sum of out-degrees and count of vertices whose value differs from `unreached`
-// (GTEPS numerator over the reached component), plus the maximum finite value.
-__global__ void reached_stats_kernel(const uint32_t *row, const uint32_t *value, uint32_t nv, uint32_t unreached,
-                                     unsigned long long *out /* [edges, vertices, max] */) {
-    unsigned long long e = 0, n = 0;
-    uint32_t mx = 0;
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
-        const uint32_t x = value[v];
-        if (x != unreached) {
-            e += __ldg(row + v + 1) - __ldg(row + v);
-            n += 1;
-            mx = max(mx, x);
-        }
-    }
-    e = dev::warp_sum(e);
-    n = dev::warp_sum(n);
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) mx = max(mx, __shfl_xor_sync(dev::kFullMask, mx, d));
-    if ((threadIdx.x & 31) == 0) {
-        if (e) atomicAdd(out, e);
-        if (n) atomicAdd(out + 1, n);
-        if (mx) atomicMax(out + 2, (unsigned long long)mx);
-    }
-}
-
 // ---------------------------------------------------------------- BC backward
 // One query over the whole cooperative grid (sg_bc.cuh has the pass itself).
 using bc::BCBackArgs;
@@ -152,29 +127,13 @@ sg_status check_graph(sg_graph *g) {
     return SG_OK;
 }
 
-// Copies a device result to the caller's buffer when it is not device memory.
+// Copies a device result to the caller's buffer when it is not device memory,
+// and with `wait` returns when it has arrived.
 template <typename T>
-sg_status deliver(sg_ctx *ctx, T *out, const T *dev_src, uint32_t n, bool out_is_dev) {
+sg_status deliver(sg_ctx *ctx, T *out, const T *dev_src, uint32_t n, bool out_is_dev, bool wait) {
     if (!out || out_is_dev) return SG_OK;
     SG_TRY_CUDA(ctx, cudaMemcpyAsync(out, dev_src, sizeof(T) * n, cudaMemcpyDeviceToHost, ctx->stream));
-    return SG_OK;
-}
-
-sg_status reached_stats(sg_graph *g, const uint32_t *value, sg_stats *stats) {
-    if (!stats) return SG_OK;
-    sg_ctx *ctx = g->ctx;
-    unsigned long long *d = nullptr;
-    SG_TRY_CUDA(ctx, sgb::graph_ws(g).get("reach_stats", 3, &d));
-    SG_TRY_CUDA(ctx, cudaMemsetAsync(d, 0, 3 * sizeof(unsigned long long), ctx->stream));
-    const int blocks = std::max(1, std::min<int>((g->nv + 255) / 256, ctx->prop.multiProcessorCount * 8));
-    reached_stats_kernel<<<blocks, 256, 0, ctx->stream>>>(g->row, value, g->nv, apps::kInf, d);
-    SG_TRY_CUDA(ctx, cudaGetLastError());
-    unsigned long long h[3];
-    SG_TRY_CUDA(ctx, cudaMemcpyAsync(h, d, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
-    SG_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    stats->edges_reached = h[0];
-    stats->vertices_reached = (uint32_t)h[1];
-    stats->search_depth = (uint32_t)h[2];
+    if (wait) SG_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return SG_OK;
 }
 
@@ -524,10 +483,10 @@ sg_status sg_bfs(sg_graph *g, uint32_t source, const sg_options *opt, uint32_t *
     SG_TRY_CUDA(ctx, sgb::graph_ws(g).get("buffer_u32", g->nv, &buffer));
     // local lookahead mixes levels inside a round, which needs the atomic minimum
     apps::BFS<uint32_t, uint32_t, graphs::NoWeight> app(source, o.non_atomic != 0 && o.local_depth <= 0);
+    cfg.reach = stats != nullptr;
     sgb::EngineResult res;
     sg_status st = sgb::run_engine<decltype(app), uint32_t, uint32_t, graphs::NoWeight>(g, app, cfg, value, buffer, &res);
-    if (st == SG_OK) st = deliver(ctx, levels_out, value, g->nv, out_dev);
-    if (st == SG_OK && cfg.blocking) st = reached_stats(g, value, stats);
+    if (st == SG_OK) st = deliver(ctx, levels_out, value, g->nv, out_dev, cfg.blocking);
     return finish(ctx, st, res, cfg, stats);
 }
 
@@ -561,10 +520,10 @@ sg_status sg_sssp(sg_graph *g, uint32_t source, const sg_options *opt, uint32_t 
         SG_TRY_CUDA(ctx, sgb::graph_ws(g).get("value_u32", g->nv, &value));
     SG_TRY_CUDA(ctx, sgb::graph_ws(g).get("buffer_u32", g->nv, &buffer));
     apps::SSSP<uint32_t, uint32_t, uint32_t> app(source);
+    cfg.reach = stats != nullptr;
     sgb::EngineResult res;
     sg_status st = sgb::run_engine<decltype(app), uint32_t, uint32_t, uint32_t>(g, app, cfg, value, buffer, &res);
-    if (st == SG_OK) st = deliver(ctx, dist_out, value, g->nv, out_dev);
-    if (st == SG_OK && cfg.blocking) st = reached_stats(g, value, stats);
+    if (st == SG_OK) st = deliver(ctx, dist_out, value, g->nv, out_dev, cfg.blocking);
     return finish(ctx, st, res, cfg, stats);
 }
 
@@ -588,16 +547,14 @@ sg_status sg_pagerank(sg_graph *g, const sg_options *opt, float *ranks_out, floa
     apps::PageRank<float, float, graphs::NoWeight> app(o.pr_error);
     sgb::EngineResult res;
     sg_status st = sgb::run_engine<decltype(app), float, float, graphs::NoWeight>(g, app, cfg, value, buffer, &res);
-    if (st == SG_OK) st = deliver(ctx, ranks_out, value, g->nv, out_dev);
-    if (st == SG_OK) st = deliver(ctx, residual_out, buffer, g->nv, res_dev);
-    if (st == SG_OK && cfg.blocking) {
-        SG_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        if (stats) {
-            stats->edges_reached = g->ne;
-            stats->vertices_reached = g->nv;
-        }
+    if (st == SG_OK) st = deliver(ctx, ranks_out, value, g->nv, out_dev, cfg.blocking);
+    if (st == SG_OK) st = deliver(ctx, residual_out, buffer, g->nv, res_dev, cfg.blocking);
+    st = finish(ctx, st, res, cfg, stats);
+    if (st == SG_OK && cfg.blocking && stats) {
+        stats->edges_reached = g->ne;
+        stats->vertices_reached = g->nv;
     }
-    return finish(ctx, st, res, cfg, stats);
+    return st;
 }
 
 sg_status sg_bc(sg_graph *g, uint32_t source, const sg_options *opt, float *bc_out, uint64_t *sigma_out,
@@ -610,6 +567,7 @@ sg_status sg_bc(sg_graph *g, uint32_t source, const sg_options *opt, float *bc_o
     sgb::EngineConfig cfg = make_config(g, o, 0, engine::LB_FINE, stats);
     if (o.lb_push < 0) cfg.lb_push = engine::LB_FINE;
     cfg.blocking = true;  // the backward pass needs the forward depth on the host
+    cfg.reach = stats != nullptr;
     const uint32_t nv = g->nv;
     const uint32_t max_levels = cfg.max_iteration + 2;
     uint32_t *level = nullptr, *buffer = nullptr, *stack = nullptr, *misc = nullptr, *ends = nullptr;
@@ -691,10 +649,10 @@ sg_status sg_bc(sg_graph *g, uint32_t source, const sg_options *opt, float *bc_o
         bc_scale_kernel<<<std::max(1u, std::min((nv + 255) / 256, 4096u)), 256, 0, ctx->stream>>>(delta, bcv, nv);
         SG_TRY_CUDA(ctx, cudaGetLastError());
     }
-    st = deliver(ctx, bc_out, bcv, nv, bc_dev);
+    st = deliver(ctx, bc_out, bcv, nv, bc_dev, false);
     if (st == SG_OK && sigma_out && !sig_dev)
         SG_TRY_CUDA(ctx, cudaMemcpyAsync(sigma_out, sigma, nv * sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx->stream));
-    if (st == SG_OK) st = reached_stats(g, level, stats);
+    SG_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     st = finish(ctx, st, res, cfg, stats);
     if (stats) {
         stats->time_total_ms = res.ms + bw_ms;

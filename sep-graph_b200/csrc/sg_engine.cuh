@@ -108,6 +108,9 @@ struct Ctrl {
     uint32_t rounds_by_variant[8];
     unsigned long long edges_processed, vertices_processed;
     unsigned long long t_start, t_end;
+    // Params::reach: out-edges, number and largest value of the reached vertices
+    unsigned long long reached_edges;
+    uint32_t reached_vertices, reached_max;
 };
 
 struct Params {
@@ -140,6 +143,8 @@ struct Params {
     // frontier neighbour within their first in-edges, and the warp form loads
     // whole lists.
     int32_t pull_coop;
+    // Sum the reached vertices (value != UINT32_MAX) when the loop ends.
+    int32_t reach;
     double alpha, beta;
     long long total_workload0;
     unsigned long long prio_init_raw, prio_step_raw;
@@ -2451,6 +2456,44 @@ struct EngineKernel {
         ps.t_round_start = dev::globaltimer_ns();
     }
 
+    // Out-edges, number and largest value of the vertices that have a value:
+    // the blocks add their shares to the control block as they leave, so the
+    // host reads them with the rest of it (a kernel, two copies and a second
+    // wait of their own took 25 of a small query's 115 us).
+    static __device__ void add_reached(const Args &a) {
+        __shared__ unsigned long long part[kWarpsPerBlock][3];
+        unsigned long long e = 0;
+        uint32_t cnt = 0, mx = 0;
+        for (uint32_t v = gthread(); v < a.csr.nnodes; v += nthreads()) {
+            const uint32_t x = (uint32_t)dev::ld_l2(a.value + v);
+            if (x != 0xffffffffu) {
+                e += out_degree(a, v);
+                cnt += 1;
+                mx = max(mx, x);
+            }
+        }
+        e = dev::warp_sum(e);
+        cnt = dev::warp_sum(cnt);
+        mx = __reduce_max_sync(dev::kFullMask, mx);
+        if (dev::lane_id() == 0) {
+            part[dev::warp_id()][0] = e;
+            part[dev::warp_id()][1] = cnt;
+            part[dev::warp_id()][2] = mx;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            unsigned long long es = 0, ns = 0, m = 0;
+            for (int w = 0; w < kWarpsPerBlock; ++w) {
+                es += part[w][0];
+                ns += part[w][1];
+                m = max(m, part[w][2]);
+            }
+            if (es) atomicAdd(&a.ctrl->reached_edges, es);
+            if (ns) atomicAdd(&a.ctrl->reached_vertices, (uint32_t)ns);
+            if (m) atomicMax(&a.ctrl->reached_max, (uint32_t)m);
+        }
+    }
+
     static __device__ void load_snap(const Args &a, Snap &s) {
         if (threadIdx.x < 4) {
             const uint4 *src = reinterpret_cast<const uint4 *>(&a.ctrl->rs);
@@ -2614,6 +2657,8 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
         }
         if (!grid_sync(c, tmo, [&] { K::leader_end_round(app, a, ps); })) return false;
     }
+    if constexpr (std::is_same<TV, uint32_t>::value)
+        if (a.p.reach) K::add_reached(a);
     if (g_team_rank == 0 && threadIdx.x == 0) {
         c->edges_processed = dev::ld_l2(&c->cnt.edges_processed);
         c->error = dev::ld_l2(&c->cnt.error);
