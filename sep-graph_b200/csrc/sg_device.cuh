@@ -187,6 +187,43 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t *queue, uint32_t *count
     return m;
 }
 
+// A warp's worklist appends of a dense phase, collected in `cap` (> 32) words
+// of shared memory and moved to the worklist with one reservation per nearly
+// `cap` items: the counter is a single word, and one returning atomic per 32
+// vertices (the 3.8 M found in one pull round of symmetric RMAT-23 took over
+// 100,000) made it the phase's bound.  All 32 lanes call every member.
+struct WarpStage {
+    uint32_t *buf;
+    uint32_t cap;
+    uint32_t *queue, *count;
+    uint32_t queue_cap;
+    uint32_t *err;
+    uint32_t n = 0;  // filled, the same in every lane
+    __device__ __forceinline__ WarpStage(uint32_t *b, uint32_t c, uint32_t *q, uint32_t *cnt, uint32_t qcap, uint32_t *e)
+        : buf(b), cap(c), queue(q), count(cnt), queue_cap(qcap), err(e) {}
+    __device__ __forceinline__ void append(bool want, uint32_t item) {
+        const uint32_t m = __ballot_sync(kFullMask, want);
+        if (want) buf[n + __popc(m & lanemask_lt())] = item;
+        n += __popc(m);
+        if (n > cap - 32) flush();
+    }
+    __device__ __forceinline__ void flush() {
+        __syncwarp();
+        if (n == 0) return;
+        uint32_t base = 0;
+        if (lane_id() == 0) base = atomicAdd(count, n);
+        base = __shfl_sync(kFullMask, base, 0);
+        for (uint32_t i = lane_id(); i < n; i += 32) {
+            if (base + i < queue_cap)
+                queue[base + i] = buf[i];
+            else
+                atomicOr(err, kErrCapacity);
+        }
+        __syncwarp();
+        n = 0;
+    }
+};
+
 // Appends, for every lane, items[k] for each set bit k (< 4) of `which`, with
 // one atomic per warp on `count`; all 32 lanes must call it.
 __device__ __forceinline__ void warp_append4(uint32_t *queue, uint32_t *count, uint32_t cap, uint32_t which,

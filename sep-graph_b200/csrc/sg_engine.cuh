@@ -538,36 +538,11 @@ struct EngineKernel {
         acc.reset();
     }
 
-    // A warp's worklist appends of a dense phase, collected in shared memory and
-    // moved to the worklist with one reservation per about 200 items: the
-    // counter is a single word, and one returning atomic per 32 vertices (the
-    // 4.6 M found in a pull round of symmetric RMAT-23 took over 100,000) made
-    // it the phase's bound.  All 32 lanes call both members.
-    struct WarpStage {
-        uint32_t *buf;  // kStageItems entries of this warp
-        uint32_t n;     // filled, the same in every lane
-        __device__ __forceinline__ void append(const Args &a, uint32_t slot, bool want, uint32_t item) {
-            const uint32_t m = __ballot_sync(dev::kFullMask, want);
-            if (want) buf[n + __popc(m & dev::lanemask_lt())] = item;
-            n += __popc(m);
-            if (n > kStageItems - 32) flush(a, slot);
-        }
-        __device__ __forceinline__ void flush(const Args &a, uint32_t slot) {
-            __syncwarp();
-            if (n == 0) return;
-            uint32_t base = 0;
-            if (dev::lane_id() == 0) base = atomicAdd(&a.ctrl->cnt.qcount[slot], n);
-            base = __shfl_sync(dev::kFullMask, base, 0);
-            for (uint32_t i = dev::lane_id(); i < n; i += 32) {
-                if (base + i < a.queue_cap)
-                    a.queue[slot][base + i] = buf[i];
-                else
-                    atomicOr(&a.ctrl->cnt.error, dev::kErrCapacity);
-            }
-            __syncwarp();
-            n = 0;
-        }
-    };
+    // Staged appends of this warp to worklist `slot`.
+    static __device__ __forceinline__ dev::WarpStage stage_for(const Args &a, uint32_t *stage, uint32_t slot) {
+        Counters *n = &a.ctrl->cnt;
+        return dev::WarpStage(stage, kStageItems, a.queue[slot], &n->qcount[slot], a.queue_cap, &n->error);
+    }
 
     // Append dst to the next worklist(s) if `want`: dedupe through the output
     // slot's queued bitmap, route by IsHighPriority when two-level priority is
@@ -1767,7 +1742,7 @@ struct EngineKernel {
         const uint32_t N = a.csr.nnodes;
         const bool natural = dev::ld_l2(&a.ctrl->cnt.middle_count) == 0;  // every vertex scheduled
         const bool split = lb != LB_NONE && a.pull_chunks;
-        WarpStage out{stage, 0};
+        dev::WarpStage out = stage_for(a, stage, s.qhi);
         const uint32_t C = split ? min(dev::ld_l2(&a.ctrl->cnt.pull_chunk_count), a.pull_chunk_cap) : 0u;
         for (uint32_t ch = gwarp(); ch < C; ch += nwarps()) {
             const uint4 c4 = __ldcg(a.pull_chunks + ch);  // the same chunk in every lane
@@ -1777,7 +1752,7 @@ struct EngineKernel {
                 want = dev::bitmap_set(a.qflag[s.qhi], c4.x);
                 if (want) count_enq(a, acc, true, c4.x);
             }
-            out.append(a, s.qhi, want, c4.x);
+            out.append(want, c4.x);
         }
         for (uint32_t base = gwarp() * 32; base < N; base += nwarps() * 32) {
             const uint32_t mw = natural ? dev::kFullMask : dev::ld_l2(a.middle + (base >> 5));
@@ -1821,11 +1796,11 @@ struct EngineKernel {
                 }
                 old = __shfl_sync(dev::kFullMask, old, 0);
                 const bool want = ((m & ~old) >> lane) & 1u;
-                out.append(a, s.qhi, want, v);
+                out.append(want, v);
                 if (want) count_enq(a, acc, true, v);
             }
         }
-        out.flush(a, s.qhi);
+        out.flush();
     }
 
     // Pull of a min-relax functor with every vertex scheduled (SSSP's pull
@@ -1853,7 +1828,7 @@ struct EngineKernel {
             const TB *offers = sync ? a.tmp : a.buffer;
             const uint32_t *bin = a.bitmap[s.bin];
             const TB none = std::numeric_limits<TB>::max();
-            WarpStage out{stage, 0};
+            dev::WarpStage out = stage_for(a, stage, s.qhi);
             for (uint32_t t = gwarp(); t < T; t += nwarps()) {
                 const uint32_t e0 = t * kPullTileEdges + lane * 8u;
                 if (lane == 0) acc.edges += min(kPullTileEdges, E - t * kPullTileEdges);
@@ -1937,12 +1912,12 @@ struct EngineKernel {
                             want = dev::bitmap_set(a.qflag[s.qhi], v);
                             if (want) count_enq(a, acc, true, v);
                         }
-                        out.append(a, s.qhi, want, v);
+                        out.append(want, v);
                     }
                     __syncwarp();  // rowbeg and rowsum are free for the next tile
                 }
             }
-            out.flush(a, s.qhi);
+            out.flush();
         }
     }
 
@@ -2223,7 +2198,7 @@ struct EngineKernel {
                 acc.active += app.App::IsActiveNode(v, dev::ld_l2(a.buffer + v));
             return;
         }
-        WarpStage out{stage, 0};
+        dev::WarpStage out = stage_for(a, stage, slot);
         for (uint32_t base = gwarp() * 32; base < N; base += nwarps() * 32) {
             const uint32_t v = base + lane;
             const bool act = v < N && app.App::IsActiveNode(v, dev::ld_l2(a.buffer + v));
@@ -2233,10 +2208,10 @@ struct EngineKernel {
             if (lane == 0) old = atomicOr(a.qflag[slot] + (base >> 5), m);
             old = __shfl_sync(dev::kFullMask, old, 0);
             const bool want = ((m & ~old) >> lane) & 1u;
-            out.append(a, slot, want, v);
+            out.append(want, v);
             if (want) count_enq(a, acc, true, v);
         }
-        out.flush(a, slot);
+        out.flush();
     }
 
     // ---------------------------------------------------------------- leader (block 0, thread 0)
