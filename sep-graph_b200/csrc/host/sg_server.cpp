@@ -148,8 +148,8 @@ sg_graph *sg_server::view(int slot, uint32_t graph_id) {
 
 uint64_t sg_server::estimate(const std::vector<Pending> &b) const {
     // Device scratch of one batch: per-team workspaces sized for the largest
-    // graph (about 32 bytes per vertex, 56 with BC's path counts, level stack
-    // and dependencies; at most one team per query and per resident block),
+    // graph (about 32 bytes per vertex, 64 with BC's path counts, level stack,
+    // dependencies and records; at most one team per query and per resident block),
     // multi-source BFS masks and level rows, and staging for host outputs.
     if (b.empty()) return 0;
     const int algo = b.front().q.algo;
@@ -162,7 +162,7 @@ uint64_t sg_server::estimate(const std::vector<Pending> &b) const {
         per_graph[p.q.graph_id]++;
     }
     const uint64_t teams = std::min<uint64_t>(b.size(), 148ull * 8);
-    uint64_t bytes = teams * nv_max * (algo == SG_QUERY_BC ? 56 : 32) + outs;
+    uint64_t bytes = teams * nv_max * (algo == SG_QUERY_BC ? 64 : 32) + outs;
     if (algo == SG_QUERY_BFS)
         for (auto &kv : per_graph)
             if (kv.second >= std::max(1u, cfg.msbfs_min))

@@ -621,6 +621,7 @@ sg_status sg_bc(sg_graph *g, uint32_t source, const sg_options *opt, float *bc_o
         ba.level = level;
         ba.sigma = sigma;
         ba.delta = delta;
+        SG_TRY_CUDA(ctx, ws.get("bc_rec", nv, &ba.rec));
         ba.bc_out = bcv;
         ba.stack = stack;
         ba.ends = ends;

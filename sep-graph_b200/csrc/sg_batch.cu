@@ -758,6 +758,7 @@ struct BCTeam {
     uint32_t *level;  // forward levels (the engine's value array)
     unsigned long long *sigma;
     float *delta;
+    uint2 *rec;
     uint32_t *stack, *ends, *misc, *ccount;  // misc: 0 stack count, 1 levels closed, 2 search depth, 3 error bits
     uint4 *chunks;
     uint32_t chunk_cap, max_levels;
@@ -853,6 +854,7 @@ __global__ void __launch_bounds__(engine::kBlockThreads)
         ba.level = bt.level;
         ba.sigma = bt.sigma;
         ba.delta = bt.delta;
+        ba.rec = bt.rec;
         ba.bc_out = outs[q];
         ba.stack = bt.stack;
         ba.ends = bt.ends;
@@ -1036,11 +1038,13 @@ sg_status prepare_batch(sg_ctx *ctx, sgb::Workspace &ws, std::vector<engine::Bat
         uint32_t *lv, *stk, *ends, *misc, *cc;
         unsigned long long *sig;
         float *dl;
+        uint2 *rec;
         uint4 *bch;
         BCTeam *dbc;
         if ((st = ws_get(ctx, ws, "bc_level", T * nv_max, &lv)) != SG_OK) return st;
         if ((st = ws_get(ctx, ws, "bc_sigma", T * nv_max, &sig)) != SG_OK) return st;
         if ((st = ws_get(ctx, ws, "bc_delta", T * nv_max, &dl)) != SG_OK) return st;
+        if ((st = ws_get(ctx, ws, "bc_rec", T * nv_max, &rec)) != SG_OK) return st;
         if ((st = ws_get(ctx, ws, "bc_stack", T * nv_max, &stk)) != SG_OK) return st;
         if ((st = ws_get(ctx, ws, "bc_ends", T * max_levels, &ends)) != SG_OK) return st;
         if ((st = ws_get(ctx, ws, "bc_ccount", T * max_levels, &cc)) != SG_OK) return st;
@@ -1048,7 +1052,7 @@ sg_status prepare_batch(sg_ctx *ctx, sgb::Workspace &ws, std::vector<engine::Bat
         if ((st = ws_get(ctx, ws, "bc_chunks", T * bchunk_cap, &bch)) != SG_OK) return st;
         std::vector<BCTeam> bts(T);
         for (size_t t = 0; t < T; ++t)
-            bts[t] = BCTeam{lv + t * nv_max, sig + t * nv_max, dl + t * nv_max, stk + t * nv_max, ends + t * max_levels,
+            bts[t] = BCTeam{lv + t * nv_max, sig + t * nv_max, dl + t * nv_max, rec + t * nv_max, stk + t * nv_max, ends + t * max_levels,
                             misc + t * 4, cc + t * max_levels, bch + t * bchunk_cap, bchunk_cap, max_levels};
         if ((st = ws_get(ctx, ws, "bc_teams", T, &dbc)) != SG_OK) return st;
         SG_TRY_CUDA(ctx, cudaMemcpyAsync(dbc, bts.data(), T * sizeof(BCTeam), cudaMemcpyHostToDevice, ctx->stream));
