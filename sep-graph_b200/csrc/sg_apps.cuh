@@ -179,6 +179,8 @@ struct PageRank : AppBase<TValue, TBuffer, TWeight> {
 
     __forceinline__ __device__ TBuffer PullReduce(TBuffer a, TBuffer b) const { return a + b; }
     __forceinline__ __device__ TBuffer PullIdentity() const { return (TBuffer)0.0f; }
+    // a push crosses the threshold exactly when the residual becomes active
+    __forceinline__ __device__ bool ActiveIsPending() const { return true; }
     // residual pushes are atomic additions: any order reaches the same fixed point within the threshold
     __forceinline__ __device__ bool ReorderSafe() const { return true; }
 };

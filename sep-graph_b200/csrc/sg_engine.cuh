@@ -379,6 +379,21 @@ template <typename App>
 struct has_pull_term<App, std::void_t<decltype(std::declval<const App &>().PullTerm(std::declval<uint32_t>()))>>
     : std::true_type {};
 
+// Optional functor extension (no reference counterpart): a PullReduce functor
+// whose vertices need scheduling exactly when IsActiveNode(buffer) holds after
+// a round's accumulations declares `bool ActiveIsPending() const` returning
+// true.  Push rounds whose worklist holds most of the edges then sum the
+// additions at the destinations (see dense_push).
+template <typename App, typename = void>
+struct has_active_is_pending : std::false_type {};
+template <typename App>
+struct has_active_is_pending<App, std::void_t<decltype(std::declval<const App &>().ActiveIsPending())>>
+    : std::true_type {};
+// A push round is dense when its worklist's out-edges are at least this share
+// (1 / kDenseShare) of all edges: a dense round costs a pass over all edges at
+// about twice the rate of the queued one.
+constexpr uint32_t kDenseShare = 2;
+
 // Edge range of chunk k of a heavy vertex's list [beg, beg + deg): chunks are
 // cut on the 4-edge grid (from beg rounded down to a multiple of 4) so that
 // every chunk starts on a 16-byte boundary of the edge arrays, which lets a
@@ -508,7 +523,51 @@ struct EngineKernel {
     // needed and the two dependent loads are skipped (the round then always
     // runs its chunk phase).
     static __device__ __forceinline__ void count_enq(const Args &a, Acc &acc, bool hi, uint32_t v) {
-        if (a.p.collect) acc.count(hi, out_degree(a, v), a.p.heavy_threshold);
+        if (a.p.collect || may_be_dense(a)) acc.count(hi, out_degree(a, v), a.p.heavy_threshold);
+    }
+
+    // Dense push rounds.  With most of the edges in the worklist, nearly every
+    // addition of a PullReduce functor is one of many to its destination: as
+    // returning atomics they are bound by the L2 atomic rate (about 50 G/s, and
+    // 56 G/s without the returned value).  Such a round combines the worklist
+    // into tmp (the identity elsewhere), sums it over the in-edges like a
+    // topology-driven pull, and rebuilds the worklist from IsActiveNode: the
+    // same additions, summed in a tree instead of one by one.  PageRank push,
+    // 1,000,003 vertices: dense rounds 290-320 -> 143 us, the call 28.9 -> 14.6 ms.
+    // Lists shorter than kDenseShare asks for stay with the queues, as do
+    // priority piles, bitmap worklists, lookahead and graphs without in-edges.
+    static __device__ __forceinline__ bool may_be_dense(const Args &a) {
+        if constexpr (has_active_is_pending<App>::value && has_pull_reduce<App, TB>::value &&
+                      std::is_same<TW, graphs::NoWeight>::value)
+            return a.tile_row && a.p.lb_push != LB_NONE && !a.p.priority && !a.p.bitmap_frontier &&
+                   a.p.local_depth == 0;
+        return false;
+    }
+    // The input slot's scout count is complete here and nobody changes it this round.
+    static __device__ __forceinline__ bool dense_push(const App &app, const Args &a, const Snap &s) {
+        if constexpr (has_active_is_pending<App>::value)
+            return may_be_dense(a) && app.ActiveIsPending() &&
+                   dev::ld_l2(&a.ctrl->cnt.scout[s.qin]) * kDenseShare >= a.csr.nedges;
+        return false;
+    }
+    // The worklist's pulled values, from its queued bits, which lose them.
+    static __device__ void combine_worklist(App &app, const Args &a, const Snap &s) {
+        if constexpr (has_pull_reduce<App, TB>::value) {
+            const uint32_t lane = dev::lane_id(), N = a.csr.nnodes;
+            uint32_t *bits = a.qflag[s.qin];
+            for (uint32_t base = gwarp() * 32; base < N; base += nwarps() * 32) {
+                const uint32_t x = dev::ld_l2(bits + (base >> 5));
+                const uint32_t v = base + lane;
+                TB out = app.PullIdentity();
+                if (v < N && ((x >> lane) & 1u)) {
+                    auto pr = app.App::CombineValueBuffer(v, a.value + v, a.buffer + v);
+                    if (pr.second) out = pr.first;
+                }
+                if (v < N) a.tmp[v] = out;
+                __syncwarp();
+                if (lane == 0 && x) bits[base >> 5] = 0;
+            }
+        }
     }
 
     // Adds the block's accumulators to the round's counters, one atomic per
@@ -2599,6 +2658,16 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
         switch (var) {
             case V_ASYNC_PUSH_DD: {
                 K::clear_dirty(a, s);
+                if (K::dense_push(app, a, s)) {
+                    K::combine_worklist(app, a, s);
+                    if (!grid_sync(c, tmo, nop)) return false;
+                    K::pull_tiles(app, a, my_lb, acc);
+                    K::flush_acc(a, acc, s.qhi, s.qlo);
+                    if (!grid_sync(c, tmo, nop)) return false;
+                    K::rebuild(app, a, s.qhi, acc, stage);
+                    K::flush_acc(a, acc, s.qhi, s.qlo);
+                    break;
+                }
                 LocalQ *lq = nullptr;
                 if (a.p.local_depth > 0 && a.p.forced == V_ASYNC_PUSH_DD && reorder_safe(app)) {
                     if (threadIdx.x == 0) {

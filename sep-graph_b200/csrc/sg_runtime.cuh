@@ -537,8 +537,10 @@ sg_status run_engine(sg_graph *g, App app, const EngineConfig &cfg, TV *value, T
     // edge-tiled topology-driven pull (functors with PullReduce): a row index per
     // 256 in-edges, found once at the launch's start
     if constexpr (has_pull_reduce<App, TB>::value && std::is_same<TW, sepgraph::graphs::NoWeight>::value) {
-        const bool td_pull = cfg.forced < 0 || cfg.forced == V_SYNC_PULL_TD;
-        if (g->has_csc && td_pull && cfg.lb_pull != LB_NONE && nv > 0)
+        // (topology-driven pull rounds, and push rounds of most of the edges)
+        const bool td_pull = (cfg.forced < 0 || cfg.forced == V_SYNC_PULL_TD) && cfg.lb_pull != LB_NONE;
+        const bool dense = has_active_is_pending<App>::value && cfg.forced == V_ASYNC_PUSH_DD && cfg.lb_push != LB_NONE;
+        if (g->has_csc && (td_pull || dense) && nv > 0)
             SG_TRY_CUDA(ctx, ws.get("pull_tiles", (ne + kPullTileEdges - 1) / kPullTileEdges + 1, &a.tile_row));
     }
     // the other pull rounds (hybrid policy or a forced pull variant): edge tiles
