@@ -770,7 +770,7 @@ using BCApp = apps::BCForward<uint32_t, uint32_t, graphs::NoWeight>;
 // same round loop as a single query) and then the backward pass over its own
 // level stack with team barriers, and writes delta * 0.5 to the query's
 // output.  Forward and backward of different queries overlap across teams.
-__global__ void __launch_bounds__(engine::kBlockThreads)
+__global__ void __launch_bounds__(engine::kBlockThreads, 4)
     batched_bc_kernel(const engine::BatchQuery<BCApp, uint32_t> *queries, uint32_t nq,
                       const engine::TeamSpace<uint32_t> *spaces, const BCTeam *bcs, float *const *outs,
                       uint32_t team_blocks, uint32_t *next_query, engine::BatchResult *results, engine::Params p) {
@@ -941,9 +941,15 @@ sg_status prepare_batch(sg_ctx *ctx, sgb::Workspace &ws, std::vector<engine::Bat
     B.bc = kBC;
     B.value_bytes = sizeof(TV);
     B.kernel = kBC ? (const void *)batched_bc_kernel : (const void *)batched_engine_kernel<App, TV, TB, TW>;
-    static std::atomic<int> occupancy{0};  // one per template instantiation
+    static std::atomic<int> occupancy[2] = {{0}, {0}};  // per template instantiation: all variants, push
+    int which = 0;
+    if constexpr (specialised<App, TB, TW>(V_ASYNC_PUSH_DD))
+        if (p.forced == V_ASYNC_PUSH_DD) {
+            B.kernel = (const void *)batched_engine_kernel<App, TV, TB, TW, V_ASYNC_PUSH_DD>;
+            which = 1;
+        }
     int max_bps = 0;
-    SG_TRY_CUDA(ctx, sgb::occupancy_once(occupancy, B.kernel, kBlockThreads, &max_bps));
+    SG_TRY_CUDA(ctx, sgb::occupancy_once(occupancy[which], B.kernel, kBlockThreads, &max_bps));
     const int bps =
         std::max(1, std::min(sgb::resident_blocks_per_sm(ctx, max_bps), o.blocks_per_sm > 0 ? o.blocks_per_sm : 4));
     const uint32_t total_blocks = (uint32_t)(ctx->prop.multiProcessorCount * bps);

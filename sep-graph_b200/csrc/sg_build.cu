@@ -600,7 +600,7 @@ struct RadixShared {
 // A warp owns 512 consecutive entries and ranks them 32 at a time, so equal
 // digits keep their order.
 template <class Source, bool kPayload>
-__global__ void __launch_bounds__(kRadixThreads)
+__global__ void __launch_bounds__(kRadixThreads, 3)  // what shared memory allows
     radix_scatter_kernel(Source in, uint64_t n, uint32_t shift, uint32_t bits, const uint32_t *base, uint32_t ntiles,
                          uint64_t *kout, uint32_t *pout) {
     extern __shared__ __align__(16) unsigned char radix_smem[];
@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(kRadixThreads)
     for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const uint64_t first = (uint64_t)t * kRadixTile + wid * (32u * kRadixItems) + lane;
         uint64_t key[kRadixItems];
-        uint32_t rank[kRadixItems];
+        uint32_t rank[kRadixItems / 2] = {};  // two 16-bit ranks each
         uint32_t valid = 0;
 #pragma unroll
         for (uint32_t r = 0; r < kRadixItems; ++r) {
@@ -630,7 +630,7 @@ __global__ void __launch_bounds__(kRadixThreads)
             __syncwarp();
             if (ok && (same & lt) == 0) sh.hist[wid][d] = before + __popc(same);
             __syncwarp();
-            rank[r] = before + __popc(same & lt);
+            rank[r / 2] |= (before + __popc(same & lt)) << (16 * (r & 1));
         }
         __syncthreads();
         {  // thread d: positions of digit d's entries in the ordered tile
@@ -664,7 +664,7 @@ __global__ void __launch_bounds__(kRadixThreads)
         for (uint32_t r = 0; r < kRadixItems; ++r) {
             if (!((valid >> r) & 1u)) continue;
             const uint32_t d = (uint32_t)(key[r] >> shift) & (bins - 1);
-            const uint32_t p = sh.hist[wid][d] + rank[r];
+            const uint32_t p = sh.hist[wid][d] + ((rank[r / 2] >> (16 * (r & 1))) & 0xffffu);
             sh.key[p] = key[r];
             if (kPayload) sh.pay[p] = in.payload(first + r * 32u);
         }

@@ -2297,10 +2297,12 @@ struct EngineKernel {
         return a.p.forced == V_SYNC_PULL_TD || a.p.forced == V_ASYNC_PUSH_TD;
     }
 
+    template <int kForced>
     static __device__ void rebuild(App &app, const Args &a, uint32_t slot, Acc &acc, uint32_t *stage) {
         const uint32_t lane = dev::lane_id();
         const uint32_t N = a.csr.nnodes;
-        if (count_only(a)) {
+        constexpr bool always = kForced == V_SYNC_PULL_TD || kForced == V_ASYNC_PUSH_TD;
+        if (always || (kForced < 0 && count_only(a))) {
             for (uint32_t v = gthread(); v < N; v += nthreads())
                 acc.active += app.App::IsActiveNode(v, dev::ld_l2(a.buffer + v));
             return;
@@ -2593,7 +2595,10 @@ struct EngineKernel {
 
 // The whole round loop of one query, run by the calling team (set_team).
 // Returns false when a bounded wait gave up (the team must stop).
-template <typename App, typename TV, typename TB, typename TW>
+// kForced = the variant of every round when it is known at compile time (the
+// forced variants that kernels are built for, see specialised), else -1: the
+// other variants' code, registers and shared memory then fall away.
+template <typename App, typename TV, typename TB, typename TW, int kForced = -1>
 __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
     using K = EngineKernel<App, TV, TB, TW>;
     __shared__ RoundState s;
@@ -2627,7 +2632,7 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
     bool tiles_listed = false;  // tile rows of a min-relax functor's pull rounds are filled
     if (reduce && a.tile_row) K::compute_tile_rows(a);
     if (!grid_sync(c, tmo, nop)) return false;
-    K::rebuild(app, a, 0, acc, stage);
+    K::template rebuild<kForced>(app, a, 0, acc, stage);
     K::flush_acc(a, acc, 0, 2);
     if (!grid_sync(c, tmo, [&] { K::leader_start(a, ps); })) return false;
 
@@ -2636,7 +2641,7 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
     for (;;) {
         K::load_snap(a, s);
         if (s.done) break;
-        const int var = s.variant;
+        const int var = kForced >= 0 ? kForced : s.variant;
         const uint32_t set = s.round & 1u;  // heavy-vertex table this round registers into
         K::set_app_variant(app, var);
         app.m_concurrent_combine =
@@ -2664,7 +2669,7 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
                     K::pull_tiles(app, a, my_lb, acc);
                     K::flush_acc(a, acc, s.qhi, s.qlo);
                     if (!grid_sync(c, tmo, nop)) return false;
-                    K::rebuild(app, a, s.qhi, acc, stage);
+                    K::template rebuild<kForced>(app, a, s.qhi, acc, stage);
                     K::flush_acc(a, acc, s.qhi, s.qlo);
                     break;
                 }
@@ -2704,7 +2709,7 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
                     K::flush_acc(a, acc, s.qhi, s.qlo);
                     if (!grid_sync(c, tmo, nop)) return false;
                 }
-                K::rebuild(app, a, s.qhi, acc, stage);
+                K::template rebuild<kForced>(app, a, s.qhi, acc, stage);
                 K::flush_acc(a, acc, s.qhi, s.qlo);
                 break;
             }
@@ -2739,7 +2744,7 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
                 K::flush_acc(a, acc, s.qhi, s.qlo);
                 if (!dd) {
                     if (!grid_sync(c, tmo, nop)) return false;
-                    K::rebuild(app, a, s.qhi, acc, stage);
+                    K::template rebuild<kForced>(app, a, s.qhi, acc, stage);
                     K::flush_acc(a, acc, s.qhi, s.qlo);
                 }
                 break;
@@ -2758,11 +2763,31 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
     return true;
 }
 
+// Forced variants with kernels of their own: delta-stepping and push PageRank
+// (ASYNC_PUSH_DD) and PageRank as topology-driven pull.  The kernel of all
+// variants needs 100 registers for SSSP and 80 for PageRank, and its rounds are
+// bound by dependent L2 trips, so the blocks it costs per SM cost time: PageRank
+// pull on RMAT-22 59.4 -> 50.9 ms, 256 SSSP in one call 51.0 -> 45.9 ms.
+template <typename App, typename TB, typename TW>
+constexpr bool specialised(int v) {
+    constexpr bool reduce = has_pull_reduce<App, TB>::value && std::is_same<TW, graphs::NoWeight>::value;
+    return (v == V_ASYNC_PUSH_DD && (reduce || has_min_relax<App, TB, TW>::value)) || (v == V_SYNC_PULL_TD && reduce);
+}
+
+// Resident blocks per SM that the kernels are compiled for (registers): the
+// unweighted functors' rounds fit 51 registers, relaxation with eight edges in
+// flight per lane takes 80 (at 64, four blocks, it spills: 256 SSSP in one call
+// 50.5 -> 55.8 ms).
+template <typename TW>
+constexpr int min_blocks() {
+    return std::is_same<TW, graphs::NoWeight>::value ? 5 : 3;
+}
+
 // One query: the whole cooperative grid is the team.
-template <typename App, typename TV, typename TB, typename TW>
-__global__ void __launch_bounds__(kBlockThreads) hybrid_engine_kernel(const App app_in, KArgs<TV, TB, TW> a) {
+template <typename App, typename TV, typename TB, typename TW, int kForced = -1>
+__global__ void __launch_bounds__(kBlockThreads, min_blocks<TW>()) hybrid_engine_kernel(const App app_in, KArgs<TV, TB, TW> a) {
     set_team(blockIdx.x, gridDim.x, a.ctrl);
-    run_instance<App, TV, TB, TW>(app_in, a);
+    run_instance<App, TV, TB, TW, kForced>(app_in, a);
 }
 
 // ---------------------------------------------------------------- batched queries
@@ -2819,8 +2844,8 @@ __device__ __forceinline__ void write_result(BatchResult *r, const Ctrl *c, uint
 // team-local barrier, records its result and moves on.  Per-query frontiers
 // and state never leave the device; the batch is one launch (capturable in a
 // CUDA graph).
-template <typename App, typename TV, typename TB, typename TW>
-__global__ void __launch_bounds__(kBlockThreads)
+template <typename App, typename TV, typename TB, typename TW, int kForced = -1>
+__global__ void __launch_bounds__(kBlockThreads, min_blocks<TW>() < 4 ? min_blocks<TW>() : 4)
     batched_engine_kernel(const BatchQuery<App, TV> *queries, uint32_t nq, const TeamSpace<TB> *spaces,
                           uint32_t team_blocks, uint32_t *next_query, BatchResult *results, Params p) {
     const uint32_t team = blockIdx.x / team_blocks;
@@ -2874,7 +2899,7 @@ __global__ void __launch_bounds__(kBlockThreads)
         if (bq.prio_raw) a.p.prio_init_raw = a.p.prio_step_raw = bq.prio_raw;
         App app = bq.app;
         app.m_p_current_round = &c->rs.round;
-        if (!run_instance<App, TV, TB, TW>(app, a)) return;
+        if (!run_instance<App, TV, TB, TW, kForced>(app, a)) return;
         if (g_team_rank == 0 && threadIdx.x == 0) write_result(results + q, c, team, 0u, c->t_end);
     }
 }

@@ -522,10 +522,21 @@ sg_status run_engine(sg_graph *g, App app, const EngineConfig &cfg, TV *value, T
     app.m_nedges = (uint32_t)ne;
     app.m_p_current_round = &a.ctrl->rs.round;
 
-    auto kernel = hybrid_engine_kernel<App, TV, TB, TW>;
-    static std::atomic<int> occupancy{0};  // one per template instantiation
+    const void *kernel = (const void *)hybrid_engine_kernel<App, TV, TB, TW>;
+    static std::atomic<int> occupancy[3] = {{0}, {0}, {0}};  // per template instantiation: all variants, push, pull
+    int which = 0;
+    if constexpr (specialised<App, TB, TW>(V_ASYNC_PUSH_DD))
+        if (cfg.forced == V_ASYNC_PUSH_DD) {
+            kernel = (const void *)hybrid_engine_kernel<App, TV, TB, TW, V_ASYNC_PUSH_DD>;
+            which = 1;
+        }
+    if constexpr (specialised<App, TB, TW>(V_SYNC_PULL_TD))
+        if (cfg.forced == V_SYNC_PULL_TD) {
+            kernel = (const void *)hybrid_engine_kernel<App, TV, TB, TW, V_SYNC_PULL_TD>;
+            which = 2;
+        }
     int max_blocks_per_sm = 0;
-    SG_TRY_CUDA(ctx, occupancy_once(occupancy, (const void *)kernel, kBlockThreads, &max_blocks_per_sm));
+    SG_TRY_CUDA(ctx, occupancy_once(occupancy[which], kernel, kBlockThreads, &max_blocks_per_sm));
     if (max_blocks_per_sm <= 0) return set_error(ctx, SG_ERR_NO_DEVICE, "engine kernel cannot be resident");
     int bps = cfg.blocks_per_sm > 0 ? cfg.blocks_per_sm : auto_blocks_per_sm(nv, ne);
     bps = std::max(1, std::min(bps, resident_blocks_per_sm(ctx, max_blocks_per_sm)));
@@ -568,7 +579,7 @@ sg_status run_engine(sg_graph *g, App app, const EngineConfig &cfg, TV *value, T
         if (window) persist_acquire(ctx);
         const bool td_pull = cfg.forced == V_SYNC_PULL_TD && a.tile_row;
         PersistWindow pw(ctx, td_pull ? (const void *)a.tmp : (const void *)a.buffer, window ? bytes : 0);
-        SG_TRY_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)kernel, grid, block, args, 0, ctx->stream));
+        SG_TRY_CUDA(ctx, cudaLaunchCooperativeKernel(kernel, grid, block, args, 0, ctx->stream));
     }
     SG_TRY_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
     if (!cfg.blocking) return SG_OK;
