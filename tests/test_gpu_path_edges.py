@@ -1,0 +1,183 @@
+"""The launch paths at the sizes where they change: hubs around the split
+thresholds of pull and backward passes, tiles with their last edge on and off
+a boundary and with few or many rows, radix passes around a tile and a digit,
+levels past the multi-source bit planes.  Against the oracle; whole numbers
+exactly, PageRank L1 <= 1e-6 (normalised, FP64 fixed point), BC 1e-4 relative
++ 1e-5 absolute as in the parity tests."""
+import numpy as np
+import pytest
+
+import oracle
+import sepgraph as sg
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = sg.Context(0)
+    yield c
+    c.close()
+
+
+def _csr(nv, s, d, w=None):
+    o = np.argsort(s, kind="stable")
+    off = np.zeros(nv + 1, np.uint32)
+    off[1:] = np.cumsum(np.bincount(s, minlength=nv))
+    return off, np.ascontiguousarray(d[o], np.uint32), None if w is None else np.ascontiguousarray(w[o], np.uint32)
+
+
+def _hub(k, tail=7):
+    """Vertex 0 -> k spokes -> one hub -> a chain; the hub has k in-edges (and, reversed, k out-edges)."""
+    spokes = np.arange(1, k + 1, dtype=np.uint32)
+    hub = k + 1
+    chain = np.arange(hub, hub + tail, dtype=np.uint32)
+    s = np.concatenate([np.zeros(k, np.uint32), spokes, chain])
+    d = np.concatenate([spokes, np.full(k, hub, np.uint32), chain + 1])
+    return hub + tail + 1, s, d
+
+
+# in-degrees around the warp threshold (32), a tile (256), the split threshold (512) and several chunks
+HUBS = [31, 32, 33, 255, 256, 257, 511, 512, 513, 1300, 5000]
+
+
+@pytest.mark.parametrize("k", HUBS)
+@pytest.mark.parametrize("variant", ["async_pull_dd", "sync_pull_dd", "auto"])
+def test_pull_into_hub(ctx, k, variant):
+    nv, s, d = _hub(k)
+    off, idx, _ = _csr(nv, s, d)
+    G = ctx.graph_from_csr(off, idx)
+    assert np.array_equal(G.bfs(0, variant=variant)[0], oracle.bfs(off, idx, 0))
+    G.close()
+    w = np.random.default_rng(k).integers(1, 64, len(s)).astype(np.uint32)
+    off, idx, w = _csr(nv, s, d, w)
+    G = ctx.graph_from_csr(off, idx, w)
+    assert np.array_equal(G.sssp(0, variant=variant)[0], oracle.sssp(off, idx, w, 0))
+    G.close()
+
+
+@pytest.mark.parametrize("k", HUBS)
+@pytest.mark.parametrize("variant", ["async_pull_dd", "async_push_dd", "auto"])
+@pytest.mark.parametrize("back", [False, True])
+def test_bc_hub(ctx, k, variant, back):
+    nv, s, d = _hub(k)
+    if back:  # the hub's k edges lead out: the backward pass sums over them
+        s, d = np.concatenate([s, d]), np.concatenate([d, s])
+    off, idx, _ = _csr(nv, s, d)
+    src = nv - 1 if back else 0
+    G = ctx.graph_from_csr(off, idx)
+    bc, sigma, _ = G.bc(src, variant=variant)
+    want, sig, _ = oracle.bc_f64(off, idx, src)
+    assert np.array_equal(sigma.astype(np.float64), sig)
+    assert np.all(np.abs(bc - want) <= 1e-4 * np.abs(want) + 1e-5)
+    bc2 = ctx.bc_batch([(G, src), (G, 0)], variant=variant)[0][0]
+    assert np.all(np.abs(bc2 - want) <= 1e-4 * np.abs(want) + 1e-5)
+    G.close()
+
+
+def _random(nv, m, seed, lo=0):
+    r = np.random.default_rng(seed)
+    return r.integers(lo, nv, m).astype(np.uint32), r.integers(lo, nv, m).astype(np.uint32)
+
+
+# edges around the 256-edge tile; vertices from one row per tile to a row per edge and mostly empty rows
+TILES = [(1, 3), (2, 255), (5, 256), (40, 257), (95, 512), (97, 513), (300, 511), (1000, 1024), (3000, 2049), (9000, 300)]
+
+
+@pytest.mark.parametrize("nv,m", TILES)
+@pytest.mark.parametrize("variant", ["async_pull_dd", "sync_pull_dd", "sync_pull_td", "auto"])
+def test_sssp_relax_tiles(ctx, nv, m, variant):
+    s, d = _random(nv, m, nv + m)
+    off, idx, w = _csr(nv, s, d, np.random.default_rng(m).integers(0, 1000, m).astype(np.uint32))
+    G = ctx.graph_from_csr(off, idx, w)
+    src = int(s[0])
+    want = oracle.sssp(off, idx, w, src)
+    assert np.array_equal(G.sssp(src, variant=variant, max_iteration=100000)[0], want)
+    other = (src + nv // 2) % nv
+    outs = ctx.sssp_batch([(G, src), (G, other)], variant=variant, max_iteration=100000)[0]
+    assert np.array_equal(outs[0], want) and np.array_equal(outs[1], oracle.sssp(off, idx, w, other))
+    G.close()
+
+
+@pytest.mark.parametrize("nv,m", TILES + [(20000, 320000)])
+@pytest.mark.parametrize("variant", ["sync_pull_td", "async_push_dd", "auto"])
+@pytest.mark.parametrize("no_csc", [False, True])
+def test_pagerank_tiles_and_dense_push(ctx, nv, m, variant, no_csc):
+    if no_csc and variant != "async_push_dd":
+        pytest.skip("pull needs the in-edge view")
+    s, d = _random(nv, m, nv * 3 + m)
+    off, idx, _ = _csr(nv, s, d)
+    want = oracle.pagerank_fixed_point_f64(off, idx)[0]
+    G = ctx.graph_from_csr(off, idx, no_csc=no_csc)
+    r = G.pagerank(variant=variant, pr_error=1e-8, max_iteration=100000)[0].astype(np.float64)
+    assert np.abs(r / r.sum() - want / want.sum()).sum() <= 1e-6
+    G.close()
+
+
+# entries around one radix tile (4096), ids around a digit (8 bits) and several
+BUILDS = [(1, 5), (2, 4095), (255, 4096), (256, 4097), (257, 8192), (65536, 8193), (65537, 20000), (70000, 3)]
+
+
+@pytest.mark.parametrize("nv,m", BUILDS)
+@pytest.mark.parametrize("code", range(8))
+@pytest.mark.parametrize("sort_rows", [False, True])
+def test_build_radix_edges(ctx, nv, m, code, sort_rows):
+    s, d = _random(nv, m, nv + 7 * m)
+    if nv > 10:
+        s[: m // 3] = 3  # one long row
+    w = np.random.default_rng(m).integers(0, 2**32, m, dtype=np.uint64).astype(np.uint32)
+    want = oracle.gtools_build(nv, s, d, w, deself_cycle=bool(code & 1), deduplicate=bool(code & 2), d2ud=bool(code & 4),
+                               sort_rows=sort_rows)
+    G = ctx.build_graph(nv, s, d, w, deself_cycle=bool(code & 1), deduplicate=bool(code & 2), d2ud=bool(code & 4),
+                        sort_rows=sort_rows)
+    off, idx, ww = G.copy_out()
+    coff, cidx, cw = G.copy_out(csc=True)
+    G.close()
+    assert all(np.array_equal(x, y) for x, y in zip((off, idx, ww), want))
+    tc = oracle.csr_tocsc(off, idx, ww)
+    assert np.array_equal(coff, tc[0]) and np.array_equal(cidx, tc[1]) and np.array_equal(cw, tc[2])
+
+
+def _cliques(n, k):
+    """A path of n cliques of k vertices: average degree about k - 1, about n levels."""
+    s, d = [], []
+    for c in range(n):
+        v = np.arange(c * k, (c + 1) * k, dtype=np.uint32)
+        a, b = np.meshgrid(v, v)
+        keep = a != b
+        s.append(a[keep]), d.append(b[keep])
+        if c:
+            s.append(np.array([c * k - 1, c * k], np.uint32)), d.append(np.array([c * k, c * k - 1], np.uint32))
+    return n * k, np.concatenate(s), np.concatenate(d)
+
+
+@pytest.mark.parametrize("n", [4, 8, 15, 30])  # up to 59 levels: below, at and past the 16 levels of the planes
+@pytest.mark.parametrize("nsrc", [1, 33, 64])
+@pytest.mark.parametrize("variant", ["auto", "async_push_dd", "async_pull_dd"])
+def test_msbfs_levels_past_planes(ctx, n, nsrc, variant):
+    nv, s, d = _cliques(n, 12)
+    off, idx, _ = _csr(nv, s, d)
+    src = np.random.default_rng(n).integers(0, nv, nsrc).astype(np.uint32)
+    src[0] = 0
+    G = ctx.graph_from_csr(off, idx, symmetric=True)
+    rows, st = G.msbfs(src, variant=variant)
+    want = np.stack([oracle.bfs(off, idx, int(x)) for x in src])
+    assert np.array_equal(rows, want)
+    for limit in (1, 3, 14, 15, 16, 17, 40):
+        rows, _ = G.msbfs(src, variant=variant, max_iteration=limit)
+        assert np.array_equal(rows, np.where(want <= limit, want, np.uint32(0xFFFFFFFF))), limit
+    G.close()
+
+
+@pytest.mark.parametrize("nv,m", [(1, 0), (3, 2), (700, 9000), (5000, 60000)])
+def test_reached_counts(ctx, nv, m):
+    s, d = _random(nv, m, nv + m)
+    off, idx, _ = _csr(nv, s, d)
+    deg = np.diff(off.astype(np.int64))
+    G = ctx.graph_from_csr(off, idx)
+    for call in (G.bfs, G.sssp):
+        val, st, _ = call(0)
+        reached = val != 0xFFFFFFFF
+        assert st.vertices_reached == reached.sum() and st.edges_reached == deg[reached].sum()
+        assert st.search_depth == val[reached].max()
+    G.close()
