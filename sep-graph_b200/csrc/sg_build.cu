@@ -20,7 +20,7 @@
 //    the radix sort needs 16 (24 with a payload), and runs when the device
 //    cannot give that.
 // Measured on B200, RMAT-21 raw weighted edges (33.5 M, self-loops and
-// duplicates dropped, rows ordered) to a CSR with its in-edge view: 9.25 ms by counting, 5.64 ms by the radix sort.
+// duplicates dropped, rows ordered) to a CSR with its in-edge view: 9.25 ms by counting, 4.25 ms by the radix sort.
 //
 // Segmented sort: rows of 2-32 keys are sorted by one warp in registers
 // (bitonic network over shuffles), rows up to 4096 keys by one block in shared
@@ -529,17 +529,22 @@ struct EdgeList {
     }
 };
 
-// What a pass reads: the edge list itself (first pass; entries that are
-// dropped report false) or the keys of the pass before.
+// What a pass reads: the edge list itself (first pass) or the keys of the pass
+// before.  raw() is the load alone, so that a thread's 16 entries are in flight
+// together; keep() then says which entries stay.
 struct EdgeSource {
     EdgeList el;
     const uint32_t *alive;  // bitmap over entries, null = all
     bool positions;         // payload = the entry's position, else its weight
-    __device__ __forceinline__ bool key(uint64_t j, uint64_t &k) const {
-        uint32_t r, c;
-        bool ok = el.entry(j, r, c);
+    __device__ __forceinline__ uint64_t raw(uint64_t j) const {
+        const uint64_t e = j >> el.rs;
+        const uint32_t a = __ldg(el.src + e), b = __ldg(el.dst + e);
+        return (j & el.rs) ? ((uint64_t)b << 32) | a : ((uint64_t)a << 32) | b;
+    }
+    __device__ __forceinline__ bool keep(uint64_t j, uint64_t k) const {
+        const uint32_t r = (uint32_t)(k >> 32), c = (uint32_t)k;
+        bool ok = !(el.deself && r == c) && r < el.nv && c < el.nv;
         if (alive) ok = ok && ((__ldg(alive + (j >> 5)) >> (j & 31)) & 1u);
-        k = ((uint64_t)r << 32) | c;
         return ok;
     }
     __device__ __forceinline__ uint32_t payload(uint64_t j) const {
@@ -553,10 +558,8 @@ struct EdgeSource {
 struct KeySource {
     const uint64_t *keys;
     const uint32_t *pay;
-    __device__ __forceinline__ bool key(uint64_t j, uint64_t &k) const {
-        k = keys[j];
-        return true;
-    }
+    __device__ __forceinline__ uint64_t raw(uint64_t j) const { return keys[j]; }
+    __device__ __forceinline__ bool keep(uint64_t, uint64_t) const { return true; }
     __device__ __forceinline__ uint32_t payload(uint64_t j) const { return pay[j]; }
     __device__ __forceinline__ void check(uint64_t, uint64_t, unsigned long long *) const {}
 };
@@ -572,13 +575,16 @@ __global__ void __launch_bounds__(kRadixThreads)
         hist[threadIdx.x] = 0;
         __syncthreads();
         const uint64_t base = (uint64_t)t * kRadixTile;
+        uint64_t key[kRadixItems];
+#pragma unroll
+        for (uint32_t k = 0; k < kRadixItems; ++k)
+            key[k] = in.raw(min(base + k * kRadixThreads + threadIdx.x, n - 1));
 #pragma unroll
         for (uint32_t k = 0; k < kRadixItems; ++k) {
             const uint64_t j = base + k * kRadixThreads + threadIdx.x;
             if (j < n) {
-                uint64_t key;
-                if (in.key(j, key)) atomicAdd(&hist[(uint32_t)(key >> shift) & (bins - 1)], 1u);
-                else in.check(j, key, first_bad);
+                if (in.keep(j, key[k])) atomicAdd(&hist[(uint32_t)(key[k] >> shift) & (bins - 1)], 1u);
+                else in.check(j, key[k], first_bad);
             }
         }
         __syncthreads();
@@ -614,10 +620,11 @@ __global__ void __launch_bounds__(kRadixThreads, 3)  // what shared memory allow
         uint32_t rank[kRadixItems / 2] = {};  // two 16-bit ranks each
         uint32_t valid = 0;
 #pragma unroll
+        for (uint32_t r = 0; r < kRadixItems; ++r) key[r] = in.raw(min(first + r * 32u, n - 1));
+#pragma unroll
         for (uint32_t r = 0; r < kRadixItems; ++r) {
-            key[r] = 0;
             const uint64_t j = first + r * 32u;
-            if (j < n && in.key(j, key[r])) valid |= 1u << r;
+            if (j < n && in.keep(j, key[r])) valid |= 1u << r;
         }
         for (uint32_t d = lane; d < kRadixBins; d += 32) sh.hist[wid][d] = 0;
         __syncwarp();
@@ -690,7 +697,10 @@ __global__ void unique_flags_kernel(const uint64_t *keys, uint64_t n, uint32_t *
     const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t w = gw; w * 32 < n; w += nw) {
         const uint64_t i = w * 32 + lane;
-        const bool first = i < n && (i == 0 || keys[i] != keys[i - 1]);
+        const uint64_t k = i < n ? keys[i] : 0;
+        uint64_t before = __shfl_up_sync(kFullMask, k, 1);
+        if (lane == 0 && i > 0 && i < n) before = keys[i - 1];
+        const bool first = i < n && (i == 0 || k != before);
         const uint32_t word = __ballot_sync(kFullMask, first);
         if (lane == 0) {
             words[w] = word;
@@ -711,8 +721,16 @@ __global__ void mark_alive_kernel(const uint32_t *pos, uint64_t n, const uint32_
 __global__ void unpack_rows_kernel(const uint64_t *keys, const uint32_t *pay, uint64_t n, const uint32_t *words,
                                    const uint32_t *wpos, uint32_t *col, uint32_t *w, uint32_t *row_begin,
                                    uint32_t *row_end) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t k = keys[i];
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    // whole warps step together: an entry's neighbours are the next lanes' keys
+    for (uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x - lane; i0 < n; i0 += step) {
+        const uint64_t i = i0 + lane;
+        const uint64_t k = i < n ? keys[i] : 0;
+        uint64_t prev = __shfl_up_sync(kFullMask, k, 1), next = __shfl_down_sync(kFullMask, k, 1);
+        if (i >= n) continue;
+        if (lane == 0 && i > 0) prev = keys[i - 1];
+        if (lane == 31 && i + 1 < n) next = keys[i + 1];
         const uint32_t row = (uint32_t)(k >> 32);
         uint32_t p = (uint32_t)i, alive = 1;
         if (words) {
@@ -724,8 +742,8 @@ __global__ void unpack_rows_kernel(const uint64_t *keys, const uint32_t *pay, ui
             col[p] = (uint32_t)k;
             if (w) w[p] = pay[i];
         }
-        if (i == 0 || (uint32_t)(keys[i - 1] >> 32) != row) row_begin[row] = p;
-        if (i + 1 == n || (uint32_t)(keys[i + 1] >> 32) != row) row_end[row] = p + alive;
+        if (i == 0 || (uint32_t)(prev >> 32) != row) row_begin[row] = p;
+        if (i + 1 == n || (uint32_t)(next >> 32) != row) row_end[row] = p + alive;
     }
 }
 
@@ -763,29 +781,29 @@ __global__ void __launch_bounds__(kRadixThreads) expand_rows_kernel(const uint32
             if (b < __ldg(row + r + 1)) mark[b > e0 ? (uint32_t)(b - e0) : 0u] = (uint32_t)(r - r0);
         }
         __syncthreads();
-        // rows ascend with the entries: a running maximum over 16 entries per thread, then over the threads
+        // rows ascend with the entries: a running maximum over each warp's 512
+        // entries, 32 at a time, then over the warps
         uint32_t m[kRadixItems], run = 0;
 #pragma unroll
         for (uint32_t k = 0; k < kRadixItems; ++k) {
-            const uint32_t x = mark[threadIdx.x * kRadixItems + k];
-            run = x > run ? x : run;
-            m[k] = run;
-        }
-        uint32_t inc = run;
+            uint32_t inc = mark[wid * (32u * kRadixItems) + k * 32u + lane];
 #pragma unroll
-        for (int s = 1; s < 32; s <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFullMask, inc, s);
-            if (lane >= (uint32_t)s) inc = max(inc, y);
+            for (int s = 1; s < 32; s <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFullMask, inc, s);
+                if (lane >= (uint32_t)s) inc = max(inc, y);
+            }
+            m[k] = max(inc, run);
+            run = __shfl_sync(kFullMask, m[k], 31);
         }
-        if (lane == 31) wmax[wid] = inc;
-        uint32_t before = __shfl_up_sync(kFullMask, inc, 1);
-        if (lane == 0) before = 0;
+        if (lane == 31) wmax[wid] = run;
         __syncthreads();
+        uint32_t before = 0;
         for (uint32_t w = 0; w < wid; ++w) before = max(before, wmax[w]);
 #pragma unroll
-        for (uint32_t k = 0; k < kRadixItems; ++k) mark[threadIdx.x * kRadixItems + k] = max(before, m[k]);
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < (uint32_t)(e1 - e0); i += kRadixThreads) src[e0 + i] = r0 + mark[i];
+        for (uint32_t k = 0; k < kRadixItems; ++k) {
+            const uint32_t i = wid * (32u * kRadixItems) + k * 32u + lane;
+            if (e0 + i < e1) src[e0 + i] = r0 + max(before, m[k]);
+        }
         __syncthreads();
     }
 }
