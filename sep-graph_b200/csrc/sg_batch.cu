@@ -829,6 +829,7 @@ __global__ void __launch_bounds__(engine::kBlockThreads, 4)
         a.ctrl = c;
         a.trace = nullptr;
         a.trace_cap = 0;
+        a.tile_row = sp.tile_row;
         a.pull_chunks = sp.pull_chunks;
         a.pull_chunk_cap = sp.pull_chunk_cap;
         a.p = p;
@@ -989,7 +990,7 @@ sg_status prepare_batch(sg_ctx *ctx, sgb::Workspace &ws, std::vector<engine::Bat
     // functors take edge tiles, the others chunks of their split destinations
     const bool pulls = (p.forced < 0 || is_pull(p.forced)) && p.lb_pull != LB_NONE;
     constexpr bool kTiles = has_min_relax<App, TB, TW>::value;
-    const size_t n_tiles = pulls && kTiles ? (ne_max + kPullTileEdges - 1) / kPullTileEdges + 1 : 0;
+    const size_t n_tiles = pulls && (kTiles || has_pull_term<App>::value) ? (ne_max + kPullTileEdges - 1) / kPullTileEdges + 1 : 0;
     const size_t n_pchunks = pulls && !kTiles ? pull_chunk_bound(ne_max) : 0;
     HeavyItem<TB> *heavy;
     Ctrl *ctrl;

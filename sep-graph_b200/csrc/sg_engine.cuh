@@ -394,6 +394,11 @@ struct has_active_is_pending<App, std::void_t<decltype(std::declval<const App &>
 // about twice the rate of the queued one.
 constexpr uint32_t kDenseShare = 2;
 
+// A pull round of such a functor goes over edge tiles when it scans at least
+// this share (1 / kTermShare) of the in-edges: an edge costs a third of what it
+// costs a thread or warp per vertex (123 M edges in 0.67 and 1.87 ms).
+constexpr uint32_t kTermShare = 3;
+
 // Edge range of chunk k of a heavy vertex's list [beg, beg + deg): chunks are
 // cut on the 4-edge grid (from beg rounded down to a multiple of 4) so that
 // every chunk starts on a 16-byte boundary of the edge arrays, which lets a
@@ -1577,7 +1582,7 @@ struct EngineKernel {
     // an atomic on one counter.  `sync` writes the combined buffer to
     // tmp (SYNC_PULL_*), else back into buffer (ASYNC_PULL_DD, algo_variants.cuh:842-849).
     // With `split`, scheduled vertices above kPullSplit in-edges list their chunks.
-    static __device__ void combine_all(App &app, const Args &a, bool sync, bool build_middle, bool split) {
+    static __device__ void combine_all(App &app, const Args &a, bool sync, bool build_middle, bool split, Acc &acc) {
         const uint32_t lane = dev::lane_id();
         const uint32_t N = a.csr.nnodes;
         bool all = true;
@@ -1591,7 +1596,7 @@ struct EngineKernel {
                 else
                     a.buffer[v] = pr.first;
                 want = pr.second;
-                if (want && split) list_pull_chunks(a, v);
+                if (want && split) list_pull_chunks(a, v, acc);
             }
             if (build_middle) {
                 const uint32_t m = __ballot_sync(dev::kFullMask, want);
@@ -1602,8 +1607,9 @@ struct EngineKernel {
         if (build_middle && !all && lane == 0) a.ctrl->cnt.middle_count = 1;  // every writer stores the same value
     }
 
-    static __device__ __forceinline__ void list_pull_chunks(const Args &a, uint32_t v) {
+    static __device__ __forceinline__ void list_pull_chunks(const Args &a, uint32_t v, Acc &acc) {
         const uint32_t beg = a.csc.begin_edge(v), deg = a.csc.end_edge(v) - beg;
+        if (has_pull_term<App>::value) acc.active += deg;  // in-edges this round scans
         if (deg <= kPullSplit) return;
         Counters *n = &a.ctrl->cnt;
         const uint32_t nch = (deg + kPullChunk - 1) / kPullChunk;
@@ -2128,6 +2134,182 @@ struct EngineKernel {
             a.tile_row[t] = (t == T || V == 0) ? (V ? V - 1 : 0) : row_of(a.csc.col_start, 0, V - 1, t * kPullTileEdges);
     }
 
+    // The rows of a tile of edges [t0, t0 + t1): segment 0 is row rlo's share,
+    // segment k the k-th row that starts inside the tile (segrow = its distance
+    // from rlo; its first edge is marked).  Returns the segments; from
+    // kPullTileRows on they are not all recorded.  All 32 lanes call.
+    static __device__ __forceinline__ uint32_t rank_tile_rows(WarpLB<TB> &w, const uint32_t *crow, uint32_t rlo,
+                                                              uint32_t rhi, uint32_t t0, uint32_t t1) {
+        const uint32_t lane = dev::lane_id();
+        if (lane < 8) w.mark[lane] = 0;
+        if (lane == 0) w.segrow[0] = 0;
+        __syncwarp();
+        uint32_t nseg = 1;
+        for (uint32_t r0 = rlo + 1; r0 <= rhi && nseg < kPullTileRows; r0 += 32) {
+            const uint32_t r = r0 + lane;
+            uint32_t at = 0;
+            bool start = false;
+            if (r <= rhi) {
+                const uint32_t b = __ldg(crow + r);
+                at = b - t0;
+                start = b < __ldg(crow + r + 1) && at < t1;  // b > t0: r is past the row of edge t0
+            }
+            const uint32_t m = __ballot_sync(dev::kFullMask, start);
+            const uint32_t k = nseg + __popc(m & dev::lanemask_lt());
+            if (start && k < kPullTileRows) {
+                w.segrow[k] = r - rlo;
+                atomicOr(&w.mark[at >> 5], 1u << (at & 31u));
+            }
+            nseg += __popc(m);
+        }
+        __syncwarp();
+        return nseg;
+    }
+
+    // Sums of the ranked segments of a tile whose edges 8 * lane .. + 7 carry
+    // g[0..7], into sums[].  All 32 lanes call.
+    template <typename T, typename Sum>
+    static __device__ __forceinline__ void segment_sums(const WarpLB<TB> &w, T *sums, const T (&g)[8], T idn,
+                                                        Sum &&sum) {
+        const uint32_t lane = dev::lane_id();
+        const uint32_t word = w.mark[lane >> 2];
+        const uint32_t heads = (word >> ((lane & 3u) * 8u)) & 0xffu;  // rows starting at this lane's edges
+        uint32_t k = 0;                                               // the segment open before this lane's edges
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j)
+            if (j < lane >> 2) k += __popc(w.mark[j]);
+        k += __popc(word & ((1u << ((lane & 3u) * 8u)) - 1u));
+        T run = idn, first = idn;
+        uint32_t seen = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if ((heads >> j) & 1u) {
+                if (seen == 0) first = run;
+                else sums[k + seen] = run;
+                run = idn;
+                ++seen;
+            }
+            run = sum(run, g[j]);
+        }
+        // sum of the open segment up to each lane's end
+        bool closed = seen != 0;
+        T open = run;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const T y = __shfl_up_sync(dev::kFullMask, open, d);
+            const uint32_t f = __shfl_up_sync(dev::kFullMask, (uint32_t)closed, d);
+            if (lane >= (uint32_t)d && !closed) {
+                open = sum(y, open);
+                closed = f != 0;
+            }
+        }
+        T before = __shfl_up_sync(dev::kFullMask, open, 1);
+        if (lane == 0) before = idn;
+        if (seen) sums[k] = sum(before, first);
+        if (lane == 31) sums[k + seen] = open;
+        __syncwarp();
+    }
+
+    // Data-driven pull of a PullTerm functor (BC's path counts) when the round
+    // scans most of the in-edges, tiled like the others: such a functor reads
+    // every in-edge of a scheduled vertex, and a thread per vertex and a warp
+    // per longer list left the lanes of a step on different lists.  Tiles
+    // without a frontier source end after the bit tests; the path counts of a
+    // row's frontier sources are summed per (row, tile).  BC on symmetric RMAT-22:
+    // its first pull round 1.87 -> 0.67 ms, the call 2.86 -> 2.34 ms.
+    static __device__ void pull_tiles_terms(App &app, const Args &a, const Snap &s, WarpLB<TB> &w, bool sync, Acc &acc,
+                                            uint32_t *stage) {
+        if constexpr (has_pull_term<App>::value) {
+            __shared__ unsigned long long sums[kWarpsPerBlock][kPullTileRows];
+            unsigned long long *segsum = sums[dev::warp_id()];
+            const uint32_t lane = dev::lane_id();
+            const uint32_t V = a.csc.nnodes, E = a.csc.nedges;
+            const uint32_t T = (E + kPullTileEdges - 1) / kPullTileEdges;
+            const uint32_t *crow = a.csc.col_start;
+            const uint32_t *srcs = a.csc.edge_source;
+            const bool aligned = (reinterpret_cast<uintptr_t>(srcs) & 15u) == 0;
+            const uint64_t pol = dev::stream_policy();
+            const TB *offers = sync ? a.tmp : a.buffer;
+            const uint32_t *bin = a.bitmap[s.bin];
+            const bool natural = dev::ld_l2(&a.ctrl->cnt.middle_count) == 0;
+            dev::WarpStage out = stage_for(a, stage, s.qhi);
+            TB offer{};  // what every frontier source offers this round, read with the first one
+            bool have_offer = false;
+            // paths into row r, by the calling lanes
+            auto deliver = [&](uint32_t r, unsigned long long paths) {
+                if (paths == 0 || !(natural || dev::bitmap_test(a.middle, r))) return false;
+                return acc_success(app.AccumulatePulled(r, a.buffer + r, offer, paths));
+            };
+            for (uint32_t t = gwarp(); t < T; t += nwarps()) {
+                const uint32_t t0 = t * kPullTileEdges, t1 = min(kPullTileEdges, E - t0);
+                const uint32_t e0 = t0 + lane * 8u;
+                uint32_t src[8];
+                if (aligned && e0 + 8u <= E) {
+                    const uint4 x = dev::ldg_v4_stream(srcs + e0, pol), y = dev::ldg_v4_stream(srcs + e0 + 4, pol);
+                    src[0] = x.x, src[1] = x.y, src[2] = x.z, src[3] = x.w;
+                    src[4] = y.x, src[5] = y.y, src[6] = y.z, src[7] = y.w;
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) src[j] = e0 + j < E ? dev::ldg_stream(srcs + e0 + j, pol) : 0u;
+                }
+                if (lane == 0) acc.edges += t1;
+                uint32_t cand = 0;
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (e0 + j < E && dev::bitmap_test_l1(bin, src[j])) cand |= 1u << j;
+                const uint32_t any = __ballot_sync(dev::kFullMask, cand != 0);
+                if (any == 0) continue;
+                unsigned long long g[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) g[j] = (cand >> j) & 1u ? app.PullTerm(src[j]) : 0ull;
+                if (!have_offer) {
+                    uint32_t u = 0;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if ((cand >> j) & 1u) u = src[j];
+                    offer = dev::ld_l2(offers + __shfl_sync(dev::kFullMask, u, __ffs(any) - 1));
+                    have_offer = true;
+                }
+                const uint32_t rlo = __ldg(a.tile_row + t), rhi = min(__ldg(a.tile_row + t + 1), V - 1);
+                const uint32_t nseg = rank_tile_rows(w, crow, rlo, rhi, t0, t1);
+                if (nseg < kPullTileRows) {
+                    segment_sums(w, segsum, g, 0ull,
+                                 [&](unsigned long long x, unsigned long long y) { return app.PullSum(x, y); });
+                    for (uint32_t q0 = 0; q0 < nseg; q0 += 32) {
+                        const uint32_t q = q0 + lane, r = q < nseg ? rlo + w.segrow[q] : rlo;
+                        bool want = q < nseg && deliver(r, segsum[q]);
+                        if (want) {
+                            dev::bitmap_set_nr(a.bitmap[s.bout], r);
+                            want = dev::bitmap_set(a.qflag[s.qhi], r);
+                            if (want) count_enq(a, acc, true, r);
+                        }
+                        out.append(want, r);
+                    }
+                } else if (cand) {  // a tile of mostly one- and two-edge rows: each lane its own
+                    uint32_t r = row_of(crow, rlo, rhi, e0);
+                    uint32_t next = __ldg(crow + r + 1);
+                    unsigned long long run = 0;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const uint32_t e = e0 + j;
+                        if ((cand >> j) & 1u) {
+                            if (e >= next) {
+                                if (deliver(r, run)) mark_pulled(a, s, r, acc);
+                                run = 0;
+                                r = row_of(crow, r + 1, rhi, e);
+                                next = __ldg(crow + r + 1);
+                            }
+                            run = app.PullSum(run, g[j]);
+                        }
+                    }
+                    if (deliver(r, run)) mark_pulled(a, s, r, acc);
+                }
+                __syncwarp();  // the segments are free for the next tile
+            }
+            out.flush();
+        }
+    }
+
     // Pull for functors with PullReduce, tiled over the in-edge array instead
     // of over destinations: a warp takes 256 consecutive CSC edges (8 per lane,
     // two 16-byte index loads, 8 independent gathers of the sources' pulled
@@ -2170,66 +2352,9 @@ struct EngineKernel {
                 TB g[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) g[j] = e0 + j < E ? dev::ld_l1(vals + s[j]) : idn;
-                // segment 0 is rlo's share of the tile, segment k the k-th row that starts inside it
-                if (lane < 8) w.mark[lane] = 0;
-                if (lane == 0) w.segrow[0] = 0;
-                __syncwarp();
-                uint32_t nseg = 1;
-                for (uint32_t r0 = rlo + 1; r0 <= rhi && nseg < kPullTileRows; r0 += 32) {
-                    const uint32_t r = r0 + lane;
-                    uint32_t at = 0;
-                    bool start = false;
-                    if (r <= rhi) {
-                        const uint32_t b = __ldg(crow + r);
-                        at = b - t0;
-                        start = b < __ldg(crow + r + 1) && at < t1;  // b > t0: r is past the row of edge t0
-                    }
-                    const uint32_t m = __ballot_sync(dev::kFullMask, start);
-                    const uint32_t k = nseg + __popc(m & dev::lanemask_lt());
-                    if (start && k < kPullTileRows) {
-                        w.segrow[k] = r - rlo;
-                        atomicOr(&w.mark[at >> 5], 1u << (at & 31u));
-                    }
-                    nseg += __popc(m);
-                }
-                __syncwarp();
+                const uint32_t nseg = rank_tile_rows(w, crow, rlo, rhi, t0, t1);
                 if (nseg < kPullTileRows) {
-                    const uint32_t word = w.mark[lane >> 2];
-                    const uint32_t heads = (word >> ((lane & 3u) * 8u)) & 0xffu;  // rows starting at this lane's edges
-                    uint32_t k = 0;  // the segment open before this lane's edges
-#pragma unroll
-                    for (uint32_t j = 0; j < 8; ++j)
-                        if (j < lane >> 2) k += __popc(w.mark[j]);
-                    k += __popc(word & ((1u << ((lane & 3u) * 8u)) - 1u));
-                    TB run = idn, first = idn;
-                    uint32_t seen = 0;
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        if ((heads >> j) & 1u) {
-                            if (seen == 0) first = run;
-                            else w.segsum[k + seen] = run;
-                            run = idn;
-                            ++seen;
-                        }
-                        run = app.PullReduce(run, g[j]);
-                    }
-                    // sum of the open segment up to each lane's end
-                    bool closed = seen != 0;
-                    TB open = run;
-#pragma unroll
-                    for (int d = 1; d < 32; d <<= 1) {
-                        const TB y = __shfl_up_sync(dev::kFullMask, open, d);
-                        const uint32_t f = __shfl_up_sync(dev::kFullMask, (uint32_t)closed, d);
-                        if (lane >= (uint32_t)d && !closed) {
-                            open = app.PullReduce(y, open);
-                            closed = f != 0;
-                        }
-                    }
-                    TB before = __shfl_up_sync(dev::kFullMask, open, 1);
-                    if (lane == 0) before = idn;
-                    if (seen) w.segsum[k] = app.PullReduce(before, first);
-                    if (lane == 31) w.segsum[k + seen] = open;
-                    __syncwarp();
+                    segment_sums(w, w.segsum, g, idn, [&](TB x, TB y) { return app.PullReduce(x, y); });
                     for (uint32_t q = lane; q < nseg; q += 32) {
                         const uint32_t r = rlo + w.segrow[q];
                         accumulate<App, TB, TW>(app, a.csc_w, r, r, 0, a.buffer + r, w.segsum[q]);
@@ -2629,7 +2754,8 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
     uint32_t *stage = &lq_block.item[0][0] + dev::warp_id() * kStageItems;  // unused while a push round runs
     constexpr bool reduce = has_pull_reduce<App, TB>::value && std::is_same<TW, graphs::NoWeight>::value;
     constexpr bool relax = has_min_relax<App, TB, TW>::value;
-    bool tiles_listed = false;  // tile rows of a min-relax functor's pull rounds are filled
+    constexpr bool terms = has_pull_term<App>::value;
+    bool tiles_listed = false;  // tile rows of a min-relax or term functor's pull rounds are filled
     if (reduce && a.tile_row) K::compute_tile_rows(a);
     if (!grid_sync(c, tmo, nop)) return false;
     K::template rebuild<kForced>(app, a, 0, acc, stage);
@@ -2723,14 +2849,18 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
                 K::release_input_flags(a, s, convert);
                 const bool reduce_td = reduce && !dd && lb_pull != LB_NONE;  // scans every vertex, no middle list
                 const bool tiles = relax && a.tile_row && lb_pull != LB_NONE && !a.p.pull_coop;
-                if (tiles && !tiles_listed) {  // read after the barrier below
+                const bool term_tiles = terms && dd && a.tile_row && a.pull_chunks && lb_pull != LB_NONE && !a.p.pull_coop;
+                if ((tiles || term_tiles) && !tiles_listed) {  // read after the barrier below
                     K::compute_tile_rows(a);
                     tiles_listed = true;
                 }
-                K::combine_all(app, a, sync, !reduce_td, !reduce_td && a.pull_chunks && lb_pull != LB_NONE);
+                K::combine_all(app, a, sync, !reduce_td, !reduce_td && a.pull_chunks && lb_pull != LB_NONE, acc);
+                if (term_tiles) K::flush_acc(a, acc, s.qhi, s.qlo);  // the in-edges to scan
                 if (!grid_sync(c, tmo, nop)) return false;
                 if (tiles && dev::ld_l2(&c->cnt.middle_count) == 0) {
                     K::pull_tiles_relax(app, a, s, my_lb, dd, sync, acc, stage);
+                } else if (term_tiles && (uint64_t)dev::ld_l2(&c->cnt.active_count) * kTermShare >= a.csc.nedges) {
+                    K::pull_tiles_terms(app, a, s, my_lb, sync, acc, stage);
                 } else if (reduce_td && a.tile_row) {
                     K::pull_tiles(app, a, my_lb, acc);
                 } else if (reduce_td) {

@@ -562,6 +562,8 @@ sg_status run_engine(sg_graph *g, App app, const EngineConfig &cfg, TV *value, T
         } else {
             a.pull_chunk_cap = (uint32_t)pull_chunk_bound(ne);
             SG_TRY_CUDA(ctx, ws.get("pull_chunks", a.pull_chunk_cap, &a.pull_chunks));
+            if constexpr (has_pull_term<App>::value)
+                SG_TRY_CUDA(ctx, ws.get("pull_tiles", (ne + kPullTileEdges - 1) / kPullTileEdges + 1, &a.tile_row));
         }
     }
 
