@@ -210,8 +210,10 @@ struct LevelStack {
         else
             atomicOr(err, dev::kErrCapacity);
     }
-    __device__ __forceinline__ void push() const {
+    // Closes a segment after `taken` more vertices.
+    __device__ __forceinline__ void push(uint32_t taken) const {
         const uint32_t n = *nlevels;
+        *count += taken;
         if (n < max_levels) {
             ends[n] = min(*count, capacity);
             *nlevels = n + 1;
@@ -228,6 +230,7 @@ struct BCForward : AppBase<TValue, TBuffer, TWeight> {
     unsigned long long *m_sigmas;
     uint32_t *m_p_search_depth;
     LevelStack m_stack;
+    uint32_t m_taken = 0;  // vertices TakeFrontier appended this round
 
     BCForward(index_t source, unsigned long long *sigmas, uint32_t *search_depth, LevelStack stack)
         : m_source_node(source), m_sigmas(sigmas), m_p_search_depth(search_depth), m_stack(stack) {}
@@ -245,7 +248,8 @@ struct BCForward : AppBase<TValue, TBuffer, TWeight> {
         if (improved) {
             *p_value = buf;
             buf += 1;
-            m_stack.append(node);
+            // data-driven rounds: TakeFrontier has it
+            if (this->m_scheduling == common::Scheduling::TOPOLOGY_DRIVEN) m_stack.append(node);
         }
         const bool schedule =
             this->m_msg_passing == MsgPassing::PUSH ? improved : (!improved && *p_buffer == kInf);
@@ -291,8 +295,25 @@ struct BCForward : AppBase<TValue, TBuffer, TWeight> {
         return buffer < prev ? this->ACCUMULATE_SUCCESS_CONTINUE : this->ACCUMULATE_FAILURE_CONTINUE;
     }
 
+    // A level-synchronous round's worklist is exactly the vertices whose level
+    // its combines fix, so the stack segment is a copy of it; appending from the
+    // combines was one reservation per 32 vertices on one counter.
+    __forceinline__ __device__ void TakeFrontier(const uint32_t *items, uint32_t n, uint32_t thread, uint32_t nthreads) {
+        const uint32_t base = dev::ld_l2(m_stack.count);  // PostComputation adds n
+        for (uint32_t i = thread; i < n; i += nthreads) {
+            if (base + i < m_stack.capacity)
+                m_stack.data[base + i] = dev::ld_l2(items + i);
+            else
+                atomicOr(m_stack.err, dev::kErrCapacity);
+        }
+        m_taken = n;
+    }
+
     __forceinline__ __device__ bool IsActiveNode(index_t, TBuffer buffer) const override { return buffer != kInf; }
-    __forceinline__ __device__ void PostComputation() override { m_stack.push(); }
+    __forceinline__ __device__ void PostComputation() override {
+        m_stack.push(m_taken);
+        m_taken = 0;
+    }
 };
 
 }  // namespace apps

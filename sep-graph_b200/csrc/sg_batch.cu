@@ -225,6 +225,7 @@ __global__ void __launch_bounds__(kMsThreads) msbfs_kernel(MsArgs a) {
         const uint4 *chunks = a.chunks[s.variant];
         if (s.variant == 0) {
             const uint32_t *act = a.active[cur];
+            dev::WarpStage out = stage_to(a.touched, &n->middle_count);
             uint32_t u4[4];
             for (uint32_t base = gw * 32; base < s.F; base += nw * 32) {
                 const uint32_t i = base + lane;
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(kMsThreads) msbfs_kernel(MsArgs a) {
                 const uint32_t steps = __reduce_max_sync(dev::kFullMask, (mine + 3u) >> 2);
                 for (uint32_t st = 0; st < steps; ++st) {
                     const uint32_t first = push4(beg + 4 * st, beg + mine, 1, f, u4);
-                    dev::warp_append4(a.touched, &n->middle_count, a.nv, first, u4, &n->error);
+                    out.append4(first, u4);
                 }
                 edges += mine;
                 uint32_t m = __ballot_sync(dev::kFullMask, mid);
@@ -254,7 +255,7 @@ __global__ void __launch_bounds__(kMsThreads) msbfs_kernel(MsArgs a) {
                     const unsigned long long fj = __shfl_sync(dev::kFullMask, f, j);
                     for (uint32_t off = 0; off < dj; off += 128) {
                         const uint32_t first = push4(bj + off + lane, bj + dj, 32, fj, u4);
-                        dev::warp_append4(a.touched, &n->middle_count, a.nv, first, u4, &n->error);
+                        out.append4(first, u4);
                     }
                     if (lane == 0) edges += dj;
                 }
@@ -265,10 +266,11 @@ __global__ void __launch_bounds__(kMsThreads) msbfs_kernel(MsArgs a) {
                 if (!f) continue;  // not in this round's frontier (the whole warp reads the same chunk)
                 for (uint32_t off = 0; off < c4.z; off += 128) {
                     const uint32_t first = push4(c4.y + off + lane, c4.y + c4.z, 32, f, u4);
-                    dev::warp_append4(a.touched, &n->middle_count, a.nv, first, u4, &n->error);
+                    out.append4(first, u4);
                 }
                 if (lane == 0) edges += c4.z;
             }
+            out.flush();
         } else {
             // pull: every vertex that misses a source ORs its in-neighbours'
             // frontier masks, stopping once every missing bit is covered: each
@@ -493,6 +495,7 @@ __global__ void __launch_bounds__(kMsThreads) msbfs_fused_kernel(MsArgs a) {
     };
     if (!engine::grid_sync(c, a.timeout_ns, start)) return;
 
+    __shared__ uint32_t stage[kMsThreads / 32][256];
     uint32_t u4[4];
     for (;;) {
         if (threadIdx.x < 4)
@@ -502,6 +505,7 @@ __global__ void __launch_bounds__(kMsThreads) msbfs_fused_kernel(MsArgs a) {
         const uint32_t p = s.qin, q = p ^ 1u;
         const bool expand = s.pile == 0;
         const uint32_t *T = a.active[p];
+        dev::WarpStage out(stage[dev::warp_id()], 256, a.active[q], &n->qcount[q], a.nv, &n->error);
         unsigned long long edges = 0;
         // OR f into up to four neighbours col[e + k * stride] (e + k * stride < end)
         // of next[q]; returns the bits k whose OR was that vertex's first (it is
@@ -555,7 +559,7 @@ __global__ void __launch_bounds__(kMsThreads) msbfs_fused_kernel(MsArgs a) {
             const uint32_t steps = __reduce_max_sync(dev::kFullMask, (mine + 3u) >> 2);
             for (uint32_t st = 0; st < steps; ++st) {
                 const uint32_t first = push4(beg + 4 * st, beg + mine, 1, nb);
-                dev::warp_append4(a.active[q], &n->qcount[q], a.nv, first, u4, &n->error);
+                out.append4(first, u4);
             }
             edges += mine;
             // larger lists: a whole warp per vertex
@@ -567,11 +571,12 @@ __global__ void __launch_bounds__(kMsThreads) msbfs_fused_kernel(MsArgs a) {
                 const unsigned long long fj = __shfl_sync(dev::kFullMask, nb, j);
                 for (uint32_t off = 0; off < dj; off += 128) {
                     const uint32_t first = push4(bj + off + lane, bj + dj, 32, fj);
-                    dev::warp_append4(a.active[q], &n->qcount[q], a.nv, first, u4, &n->error);
+                    out.append4(first, u4);
                 }
                 if (lane == 0) edges += dj;
             }
         }
+        out.flush();
         edges = dev::warp_sum(edges);
         if (lane == 0 && edges) atomicAdd(&n->edges_processed, edges);
         auto end_round = [&] {

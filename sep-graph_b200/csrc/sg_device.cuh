@@ -207,6 +207,24 @@ struct WarpStage {
         n += __popc(m);
         if (n > cap - 32) flush();
     }
+    // Every lane appends items[k] for each set bit k (< 4) of `which`; cap >= 128.
+    __device__ __forceinline__ void append4(uint32_t which, const uint32_t (&items)[4]) {
+        if (!__any_sync(kFullMask, which != 0)) return;
+        const uint32_t c = __popc(which);
+        uint32_t incl = c;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFullMask, incl, d);
+            if (lane_id() >= (uint32_t)d) incl += y;
+        }
+        const uint32_t total = __shfl_sync(kFullMask, incl, 31);
+        if (n + total > cap) flush();
+        uint32_t pos = n + incl - c;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if ((which >> k) & 1u) buf[pos++] = items[k];
+        n += total;
+    }
     __device__ __forceinline__ void flush() {
         __syncwarp();
         if (n == 0) return;
@@ -223,34 +241,6 @@ struct WarpStage {
         n = 0;
     }
 };
-
-// Appends, for every lane, items[k] for each set bit k (< 4) of `which`, with
-// one atomic per warp on `count`; all 32 lanes must call it.
-__device__ __forceinline__ void warp_append4(uint32_t *queue, uint32_t *count, uint32_t cap, uint32_t which,
-                                             const uint32_t (&items)[4], uint32_t *err) {
-    const uint32_t c = __popc(which);
-    uint32_t incl = c;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t y = __shfl_up_sync(kFullMask, incl, d);
-        if (lane_id() >= (uint32_t)d) incl += y;
-    }
-    const uint32_t total = __shfl_sync(kFullMask, incl, 31);
-    if (total == 0) return;
-    uint32_t base = 0;
-    if (lane_id() == 31) base = atomicAdd(count, total);
-    base = __shfl_sync(kFullMask, base, 31);
-    uint32_t pos = base + incl - c;
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        if ((which >> k) & 1u) {
-            if (pos < cap)
-                queue[pos] = items[k];
-            else
-                atomicOr(err, kErrCapacity);
-            ++pos;
-        }
-}
 
 __device__ __forceinline__ bool bitmap_test(const uint32_t *bm, uint32_t v) {
     return (ld_l2(bm + (v >> 5)) >> (v & 31u)) & 1u;
@@ -269,6 +259,9 @@ __device__ __forceinline__ void bitmap_clear(uint32_t *bm, uint32_t v) { atomicA
 // the issuing thread never waits for.
 __device__ __forceinline__ void bitmap_set_nr(uint32_t *bm, uint32_t v) {
     asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" ::"l"(bm + (v >> 5)), "r"(1u << (v & 31u)) : "memory");
+}
+__device__ __forceinline__ void bitmap_and_nr(uint32_t *word, uint32_t bits) {
+    asm volatile("red.relaxed.gpu.global.and.b32 [%0], %1;" ::"l"(word), "r"(bits) : "memory");
 }
 __device__ __forceinline__ void bitmap_or_nr(uint32_t *word, uint32_t bits) {
     asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" ::"l"(word), "r"(bits) : "memory");

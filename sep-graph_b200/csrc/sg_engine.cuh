@@ -245,10 +245,14 @@ struct WarpLB {
             uint32_t mark[8];
         };
     };
+    // topology-driven pull without tiles: each lane's first and last (possibly shared) segment
+    __device__ __forceinline__ uint32_t *partk(int k) { return heavy_src + 32 * k; }
+    __device__ __forceinline__ TBuffer *part(int k) { return heavy_pay + 32 * k; }
     TBuffer pay[32];
-    // topology-driven pull: each lane's first and last (possibly shared) segment
-    uint32_t partk[2][32];
-    TBuffer part[2][32];
+    // push rounds: heavy vertices not registered yet (see stage_heavy)
+    uint32_t heavy_n, heavy_src[64], heavy_beg[64], heavy_deg[64];
+    TBuffer heavy_pay[64];
+    uint32_t far_item[64];  // far pile: vertices taken and not processed yet
     // edge-tiled pull of min-relax functors: per-row minima of one tile
     TBuffer rowsum[kPullTileRows];
     // bitmap worklist: exclusive scan of the lanes' set bits
@@ -275,11 +279,19 @@ struct Acc {
     uint32_t heavy_hi, heavy_lo;
     unsigned long long edges;
     uint32_t active;
+    uint32_t push_hi, push_lo;  // bits set in a bitmap worklist / the far pile (or left in it)
+    uint32_t popped;
+    // This warp's staged appends to the near worklist (push rounds without
+    // lookahead): kStageItems entries, the first stage_n filled (the same in
+    // every lane); null = every append reserves its own entries.
+    uint32_t *stage;
+    uint32_t stage_n;
     __device__ void reset() {
         scout_hi = scout_lo = 0;
         heavy_hi = heavy_lo = 0;
         edges = 0;
         active = 0;
+        push_hi = push_lo = popped = 0;
     }
     __device__ __forceinline__ void count(bool hi, uint32_t deg, uint32_t heavy_threshold) {
         const uint32_t h = deg > heavy_threshold;
@@ -398,6 +410,17 @@ constexpr uint32_t kDenseShare = 2;
 // this share (1 / kTermShare) of the in-edges: an edge costs a third of what it
 // costs a thread or warp per vertex (123 M edges in 0.67 and 1.87 ms).
 constexpr uint32_t kTermShare = 3;
+
+// Optional functor extension (no reference counterpart): a functor that keeps
+// the vertices of every data-driven round declares
+//   __device__ void TakeFrontier(const index_t *items, uint32_t n, uint32_t thread, uint32_t nthreads)
+// called by all threads of the team before the round's combines with its input
+// worklist (each vertex once; thread = 0 .. nthreads - 1).
+template <typename App, typename = void>
+struct has_take_frontier : std::false_type {};
+template <typename App>
+struct has_take_frontier<App, std::void_t<decltype(std::declval<App &>().TakeFrontier(
+                                  std::declval<const uint32_t *>(), 0u, 0u, 0u))>> : std::true_type {};
 
 // Edge range of chunk k of a heavy vertex's list [beg, beg + deg): chunks are
 // cut on the 4-edge grid (from beg rounded down to a multiple of 4) so that
@@ -576,22 +599,31 @@ struct EngineKernel {
     }
 
     // Adds the block's accumulators to the round's counters, one atomic per
-    // block and counter: all blocks update the same few words, and an atomic
-    // per warp (up to 9,472 warps) queued behind one L2 slice at every phase
-    // end.  All threads of the block call, and the next call comes after a
-    // block barrier (every phase ends in a grid barrier).
+    // block and counter: all blocks update the same few words, one word takes an
+    // atomic only every 2.5 to 5 ns, and an atomic per warp (up to 9,472 warps)
+    // or per step of a warp queued for longer than the phase's work took:
+    // delta-stepping on RMAT-22, the round over 35 M hub edges 613 -> 266 us.  All
+    // threads of the block call, and the next call comes after a block barrier
+    // (every phase ends in a grid barrier).
     static __device__ void flush_acc(const Args &a, Acc &acc, uint32_t q_hi, uint32_t q_lo) {
-        __shared__ unsigned long long part[kWarpsPerBlock][6];
-        unsigned long long x[6] = {dev::warp_sum(acc.scout_hi), dev::warp_sum(acc.scout_lo),
-                                   (unsigned long long)dev::warp_sum(acc.heavy_hi),
-                                   (unsigned long long)dev::warp_sum(acc.heavy_lo), dev::warp_sum(acc.edges),
-                                   (unsigned long long)dev::warp_sum(acc.active)};
-        if (dev::lane_id() == 0) {
+        constexpr int kSums = 9;
+        __shared__ unsigned long long part[kWarpsPerBlock][kSums];
+        if (acc.stage) flush_stage(a, acc, q_hi);
+        const unsigned long long wide[3] = {acc.scout_hi, acc.scout_lo, acc.edges};
+        const uint32_t narrow[6] = {acc.heavy_hi, acc.heavy_lo, acc.active, acc.push_hi, acc.push_lo, acc.popped};
 #pragma unroll
-            for (int k = 0; k < 6; ++k) part[dev::warp_id()][k] = x[k];
+        for (int k = 0; k < 3; ++k) {
+            unsigned long long x = 0;
+            if (__any_sync(dev::kFullMask, wide[k] != 0)) x = dev::warp_sum(wide[k]);
+            if (dev::lane_id() == 0) part[dev::warp_id()][k] = x;
+        }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            const uint32_t x = __reduce_add_sync(dev::kFullMask, narrow[k]);
+            if (dev::lane_id() == 0) part[dev::warp_id()][3 + k] = x;
         }
         __syncthreads();
-        if (threadIdx.x < 6) {
+        if (threadIdx.x < kSums) {
             const uint32_t k = threadIdx.x;
             unsigned long long sum = 0;
 #pragma unroll
@@ -599,12 +631,49 @@ struct EngineKernel {
             Counters *n = &a.ctrl->cnt;
             if (sum) {
                 if (k < 2) atomicAdd(&n->scout[k == 0 ? q_hi : q_lo], sum);
-                else if (k < 4) atomicAdd(&n->heavy_enq[k == 2 ? q_hi : q_lo], (uint32_t)sum);
-                else if (k == 4) atomicAdd(&n->edges_processed, sum);
-                else atomicAdd(&n->active_count, (uint32_t)sum);
+                else if (k == 2) atomicAdd(&n->edges_processed, sum);
+                else if (k < 5) atomicAdd(&n->heavy_enq[k == 3 ? q_hi : q_lo], (uint32_t)sum);
+                else if (k == 5) atomicAdd(&n->active_count, (uint32_t)sum);
+                else if (k < 8) atomicAdd(&n->qcount[k == 6 ? q_hi : q_lo], (uint32_t)sum);
+                else atomicAdd(&n->popped, (uint32_t)sum);
             }
         }
         acc.reset();
+    }
+
+    // Moves the warp's staged appends to worklist `slot` with one reservation.
+    static __device__ __forceinline__ void flush_stage(const Args &a, Acc &acc, uint32_t slot) {
+        if (acc.stage_n == 0) return;
+        Counters *n = &a.ctrl->cnt;
+        __syncwarp();
+        uint32_t base = 0;
+        if (dev::lane_id() == 0) base = atomicAdd(&n->qcount[slot], acc.stage_n);
+        base = __shfl_sync(dev::kFullMask, base, 0);
+        for (uint32_t i = dev::lane_id(); i < acc.stage_n; i += 32) {
+            if (base + i < a.queue_cap)
+                a.queue[slot][base + i] = acc.stage[i];
+            else
+                atomicOr(&n->error, dev::kErrCapacity);
+        }
+        __syncwarp();
+        acc.stage_n = 0;
+    }
+
+    // The position of this lane's `c` appends to worklist `slot`, `total` of
+    // the warp's, `before` of the lower lanes': in the stage (returns true) or,
+    // without one, reserved in the worklist.
+    static __device__ __forceinline__ bool place(const Args &a, Acc &acc, uint32_t slot, uint32_t total, uint32_t before,
+                                                 uint32_t *pos) {
+        if (acc.stage) {
+            if (acc.stage_n + total > kStageItems) flush_stage(a, acc, slot);
+            *pos = acc.stage_n + before;
+            acc.stage_n += total;
+            return true;
+        }
+        uint32_t base = 0;
+        if (dev::lane_id() == 0) base = atomicAdd(&a.ctrl->cnt.qcount[slot], total);
+        *pos = __shfl_sync(dev::kFullMask, base, 0) + before;
+        return false;
     }
 
     // Staged appends of this warp to worklist `slot`.
@@ -646,31 +715,39 @@ struct EngineKernel {
             }
             want = want && !loc;
         }
-        bool w_hi = want && hi, w_lo = want && !hi;
+        bool w_hi = want && hi;
+        const bool w_lo = want && !hi;
+        if (w_lo) {  // the far pile is a bitmap (see push_far)
+            dev::bitmap_set_nr(a.qflag[s.qlo], dst);
+            ++acc.push_lo;
+        }
         if (a.p.bitmap_frontier) {
             // no dedupe round trip and no append: the bit is the worklist entry
-            if (w_hi) dev::bitmap_set_nr(a.qflag[s.qhi], dst);
-            if (w_lo) dev::bitmap_set_nr(a.qflag[s.qlo], dst);
-            count_pushes(n, s, w_hi, w_lo);
-            if (w_hi || w_lo) count_enq(a, acc, w_hi, dst);
-            return;
+            if (w_hi) {
+                dev::bitmap_set_nr(a.qflag[s.qhi], dst);
+                ++acc.push_hi;
+            }
+        } else {
+            if (w_hi) w_hi = dev::bitmap_set(a.qflag[s.qhi], dst);
+            const uint32_t m = __ballot_sync(dev::kFullMask, w_hi);
+            if (m) {
+                uint32_t pos;
+                const bool staged = place(a, acc, s.qhi, __popc(m), __popc(m & dev::lanemask_lt()), &pos);
+                if (w_hi) put(a, acc, s.qhi, staged, pos, dst);
+                __syncwarp();
+            }
         }
-        if (w_hi) w_hi = dev::bitmap_set(a.qflag[s.qhi], dst);
-        if (w_lo) w_lo = dev::bitmap_set(a.qflag[s.qlo], dst);
-        dev::warp_append(a.queue[s.qhi], &n->qcount[s.qhi], a.queue_cap, w_hi, dst, &n->error);
-        if (a.p.priority) dev::warp_append(a.queue[s.qlo], &n->qcount[s.qlo], a.queue_cap, w_lo, dst, &n->error);
         if (w_hi || w_lo) count_enq(a, acc, w_hi, dst);
     }
 
-    // Bitmap worklists: one fire-and-forget add per warp and slot of the
-    // number of pushes (the leader only needs to know whether a slot is empty).
-    // All 32 lanes must call.
-    static __device__ __forceinline__ void count_pushes(Counters *n, const Snap &s, bool w_hi, bool w_lo) {
-        const uint32_t mh = __ballot_sync(dev::kFullMask, w_hi), ml = __ballot_sync(dev::kFullMask, w_lo);
-        if (dev::lane_id() == 0) {
-            if (mh) dev::red_add(&n->qcount[s.qhi], (uint32_t)__popc(mh));
-            if (ml) dev::red_add(&n->qcount[s.qlo], (uint32_t)__popc(ml));
-        }
+    static __device__ __forceinline__ void put(const Args &a, Acc &acc, uint32_t slot, bool staged, uint32_t pos,
+                                               uint32_t v) {
+        if (staged)
+            acc.stage[pos] = v;
+        else if (pos < a.queue_cap)
+            a.queue[slot][pos] = v;
+        else
+            atomicOr(&a.ctrl->cnt.error, dev::kErrCapacity);
     }
 
     // K pushes per lane at once, with the candidate values the pushes offer
@@ -712,54 +789,43 @@ struct EngineKernel {
                 want[j] = want[j] && !loc;
             }
         }
-        if (a.p.bitmap_frontier) {
-            uint32_t ch = 0, cl = 0;
-#pragma unroll
-            for (int j = 0; j < K; ++j) {
-                if (want[j]) {
-                    dev::bitmap_set_nr(a.qflag[hi[j] ? s.qhi : s.qlo], dst[j]);
-                    count_enq(a, acc, hi[j], dst[j]);
-                }
-                ch += want[j] && hi[j];
-                cl += want[j] && !hi[j];
-            }
-            ch = dev::warp_sum(ch);
-            cl = dev::warp_sum(cl);
-            if (dev::lane_id() == 0) {
-                if (ch) dev::red_add(&n->qcount[s.qhi], ch);
-                if (cl) dev::red_add(&n->qcount[s.qlo], cl);
-            }
-            return;
-        }
         bool w[K];
-#pragma unroll
-        for (int j = 0; j < K; ++j) w[j] = want[j] ? dev::bitmap_set(a.qflag[hi[j] ? s.qhi : s.qlo], dst[j]) : false;
-        uint32_t ch = 0, cl = 0;
+        uint32_t ch = 0;
 #pragma unroll
         for (int j = 0; j < K; ++j) {
-            ch += w[j] && hi[j];
-            cl += w[j] && !hi[j];
+            w[j] = want[j] && hi[j];
+            if (want[j] && !hi[j]) {  // far pile: the bit is the entry
+                dev::bitmap_set_nr(a.qflag[s.qlo], dst[j]);
+                count_enq(a, acc, false, dst[j]);
+                ++acc.push_lo;
+            }
         }
-        const uint32_t ih = dev::warp_inclusive_scan(ch), il = dev::warp_inclusive_scan(cl);
-        const uint32_t th = __shfl_sync(dev::kFullMask, ih, 31), tl = __shfl_sync(dev::kFullMask, il, 31);
-        uint32_t bh = 0, bl = 0;
-        if (dev::lane_id() == 0) {
-            if (th) bh = atomicAdd(&n->qcount[s.qhi], th);
-            if (tl) bl = atomicAdd(&n->qcount[s.qlo], tl);
+        if (a.p.bitmap_frontier) {
+#pragma unroll
+            for (int j = 0; j < K; ++j)
+                if (w[j]) {
+                    dev::bitmap_set_nr(a.qflag[s.qhi], dst[j]);
+                    count_enq(a, acc, true, dst[j]);
+                    ++acc.push_hi;
+                }
+            return;
         }
-        bh = __shfl_sync(dev::kFullMask, bh, 0) + ih - ch;
-        bl = __shfl_sync(dev::kFullMask, bl, 0) + il - cl;
+#pragma unroll
+        for (int j = 0; j < K; ++j)
+            if (w[j]) w[j] = dev::bitmap_set(a.qflag[s.qhi], dst[j]);
+#pragma unroll
+        for (int j = 0; j < K; ++j) ch += w[j];
+        if (!__any_sync(dev::kFullMask, ch != 0)) return;
+        const uint32_t ih = dev::warp_inclusive_scan(ch);
+        uint32_t pos;
+        const bool staged = place(a, acc, s.qhi, __shfl_sync(dev::kFullMask, ih, 31), ih - ch, &pos);
 #pragma unroll
         for (int j = 0; j < K; ++j) {
             if (!w[j]) continue;
-            const uint32_t q = hi[j] ? s.qhi : s.qlo;
-            const uint32_t pos = hi[j] ? bh++ : bl++;
-            if (pos < a.queue_cap)
-                a.queue[q][pos] = dst[j];
-            else
-                atomicOr(&n->error, dev::kErrCapacity);
-            count_enq(a, acc, hi[j], dst[j]);
+            put(a, acc, s.qhi, staged, pos++, dst[j]);
+            count_enq(a, acc, true, dst[j]);
         }
+        __syncwarp();
     }
 
     // Single-thread enqueue (LB NONE paths run divergent per-thread loops).
@@ -776,14 +842,56 @@ struct EngineKernel {
                 return;
             }
         }
-        const uint32_t q = hi ? s.qhi : s.qlo;
-        if (!dev::bitmap_set(a.qflag[q], dst)) return;
-        const uint32_t pos = atomicAdd(&n->qcount[q], 1u);
+        if (!hi) {  // far pile: the bit is the entry
+            dev::bitmap_set_nr(a.qflag[s.qlo], dst);
+            ++acc.push_lo;
+            count_enq(a, acc, false, dst);
+            return;
+        }
+        if (!dev::bitmap_set(a.qflag[s.qhi], dst)) return;
+        const uint32_t pos = atomicAdd(&n->qcount[s.qhi], 1u);
         if (pos < a.queue_cap)
-            a.queue[q][pos] = dst;
+            a.queue[s.qhi][pos] = dst;
         else
             atomicOr(&n->error, dev::kErrCapacity);
         count_enq(a, acc, hi, dst);
+    }
+
+    // A push step's heavy vertices, kept in shared memory until 32 of them share
+    // the table's two reservations (its counters are single words too).  All 32
+    // lanes call; flush_heavy registers what is left at the phase's end.
+    static __device__ __forceinline__ void stage_heavy(const Args &a, WarpLB<TB> &w, uint32_t set, bool heavy,
+                                                       uint32_t src, uint32_t beg, uint32_t deg, TB payload) {
+        const uint32_t m = __ballot_sync(dev::kFullMask, heavy);
+        if (m == 0) return;
+        uint32_t n = w.heavy_n;
+        if (heavy) {
+            const uint32_t k = n + __popc(m & dev::lanemask_lt());
+            w.heavy_src[k] = src;
+            w.heavy_beg[k] = beg;
+            w.heavy_deg[k] = deg;
+            w.heavy_pay[k] = payload;
+        }
+        n += __popc(m);
+        __syncwarp();
+        if (n >= 32) {
+            n -= 32;  // the newest 32 go, the older ones stay in front
+            const uint32_t k = n + dev::lane_id();
+            register_heavy(a, set, true, w.heavy_src[k], w.heavy_beg[k], w.heavy_deg[k], w.heavy_pay[k]);
+            __syncwarp();
+        }
+        if (dev::lane_id() == 0) w.heavy_n = n;
+        __syncwarp();
+    }
+    static __device__ __forceinline__ void flush_heavy(const Args &a, WarpLB<TB> &w, uint32_t set) {
+        const uint32_t n = w.heavy_n, k = dev::lane_id();
+        if (n == 0) return;
+        const bool in = k < n;
+        register_heavy(a, set, in, in ? w.heavy_src[k] : 0u, in ? w.heavy_beg[k] : 0u, in ? w.heavy_deg[k] : 0u,
+                       in ? w.heavy_pay[k] : TB{});
+        __syncwarp();
+        if (k == 0) w.heavy_n = 0;
+        __syncwarp();
     }
 
     // Registers the lanes' heavy vertices as chunk lists (warp-aggregated: one
@@ -1381,7 +1489,9 @@ struct EngineKernel {
         const uint32_t lane = dev::lane_id();
         const uint32_t N = dd ? s.F : a.csr.nnodes;
         const uint32_t *Q = a.queue[s.qin];
-        if (dd && a.p.bitmap_frontier) {
+        if (dd && s.pile) {
+            push_far(app, a, s, wlb, lb, acc, lq);
+        } else if (dd && a.p.bitmap_frontier) {
             // The worklist is the input slot's bitmap.  A warp takes 32 x 8 words
             // spread evenly over the vertex range (word gw + k * nwarps), so every
             // warp samples every region of the id space (RMAT graphs put their
@@ -1440,8 +1550,7 @@ struct EngineKernel {
                 }
                 __syncwarp();
             }
-            popped = dev::warp_sum(popped);
-            if (lane == 0 && popped) dev::red_add(&a.ctrl->cnt.popped, popped);
+            acc.popped += popped;
         } else {
             for (uint32_t base = gwarp() * 32; base < N; base += nwarps() * 32) {
                 const uint32_t i = base + lane;
@@ -1451,44 +1560,97 @@ struct EngineKernel {
                 push_item(app, a, s, wlb, dd, lb, acc, lq, v, valid, dd);
             }
         }
+        flush_heavy(a, wlb, s.round & 1u);
         if (lq) local_levels(app, a, s, wlb, lb, acc, lq);
     }
 
-    // One worklist item per lane (valid lanes): pop (queue worklists), far-pile
-    // check, combine, heavy registration and the warp's expansion.  All 32
+    // The far pile of two-level priority: one bitmap (slot qlo) for the whole
+    // run.  A push outside the window sets its vertex's bit with a reduction and
+    // appends nothing; when the near pile has drained and the window has moved
+    // on, every warp takes words spread over the vertex range, reads the values
+    // of a word's vertices with one coalesced load, clears the bits of those
+    // that are now inside the window and processes them 32 at a time.  The
+    // others simply stay set, where a pile kept as a queue was read at random,
+    // deduplicated and appended again every time the window moved.  Delta-stepping
+    // on RMAT-22, the window's moves over about a million far vertices 103 / 64 /
+    // 47 us -> 83 / 46 / 31 us.
+    // A vertex's bit is cleared before the vertex is combined.  A min-relax
+    // functor needs no fence in between: no push from outside the window can
+    // lower a vertex whose value is inside it, so nobody sets the bit again.
+    static __device__ void push_far(App &app, const Args &a, const Snap &s, WarpLB<TB> &w, int lb, Acc &acc,
+                                    LocalQ *lq) {
+        const uint32_t lane = dev::lane_id();
+        const TB prio = from_raw<TB>(s.prio_raw);
+        uint32_t *bits = a.qflag[s.qlo];
+        uint32_t *buf = w.far_item;
+        const uint32_t W = a.nwords, nw = nwarps();
+        uint32_t n = 0, kept = 0, popped = 0;
+        for (uint64_t b = gwarp(); b < W; b += (uint64_t)32 * nw) {
+            const uint64_t wi = b + (uint64_t)lane * nw;
+            const uint32_t x = wi < W ? dev::ld_l2(bits + wi) : 0u;
+            uint32_t left = __ballot_sync(dev::kFullMask, x != 0);
+            uint32_t gone = 0;  // taken bits of this lane's word
+            while (left) {      // four words' values in flight
+                uint32_t j[4], tm[4], v[4];
+                bool in[4];
+                TB val[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    j[q] = left ? (uint32_t)__ffs(left) - 1 : 32u;
+                    left &= left - 1;
+                    const uint32_t xq = __shfl_sync(dev::kFullMask, x, j[q] & 31u);
+                    in[q] = j[q] < 32u && ((xq >> lane) & 1u);
+                    v[q] = (uint32_t)(b + (uint64_t)j[q] * nw) * 32u + lane;
+                    val[q] = in[q] ? dev::ld_l2(a.buffer + v[q]) : TB{};
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    in[q] = in[q] && app.App::IsHighPriority(prio, val[q]);
+                    tm[q] = __ballot_sync(dev::kFullMask, in[q]);
+                    if (lane == j[q] && tm[q]) {
+                        gone = tm[q];
+                        dev::bitmap_and_nr(bits + wi, ~gone);
+                    }
+                }
+                if constexpr (!has_min_relax<App, TB, TW>::value) __threadfence();
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (in[q]) buf[n + __popc(tm[q] & dev::lanemask_lt())] = v[q];
+                    n += __popc(tm[q]);
+                    __syncwarp();
+                    if (n >= 32) {
+                        const uint32_t item = buf[lane];
+                        n -= 32;
+                        const uint32_t rest = lane < n ? buf[32 + lane] : 0u;
+                        __syncwarp();
+                        buf[lane] = rest;
+                        push_item(app, a, s, w, true, lb, acc, lq, item, true, false);
+                        __syncwarp();
+                    }
+                }
+            }
+            kept += __popc(x & ~gone);
+            popped += __popc(gone);
+        }
+        if (n) push_item(app, a, s, w, true, lb, acc, lq, lane < n ? buf[lane] : 0u, lane < n, false);
+        acc.push_lo += kept;
+        acc.popped += popped;
+    }
+
+    // One worklist item per lane (valid lanes): pop (queue worklists), combine,
+    // heavy registration and the warp's expansion.  All 32
     // lanes must call.
     static __device__ __forceinline__ void push_item(App &app, const Args &a, const Snap &s, WarpLB<TB> &wlb,
                                                      bool dd, int lb, Acc &acc, LocalQ *lq, uint32_t v, bool valid,
                                                      bool pop) {
         const TB prio = from_raw<TB>(s.prio_raw);
-        Counters *n = &a.ctrl->cnt;
         {
             bool proceed = valid;
-            bool keep = false;
             if (valid) {
                 // sampling priority: a topology-driven round takes only the
                 // vertices above this round's sampled threshold (driver.cuh:362-383)
                 if (!dd && a.p.sample_cut > 0.f) proceed = app.App::IsHighPriority(prio, dev::ld_l2(a.buffer + v));
-                if (dd) {
-                    if (pop) dev::bitmap_clear(a.qflag[s.qin], v);  // pop
-                    if (s.pile && !app.App::IsHighPriority(prio, dev::ld_l2(a.buffer + v))) {
-                        // far pile: vertices still outside the priority window move to the new pile
-                        if (a.p.bitmap_frontier) {
-                            dev::bitmap_set_nr(a.qflag[s.qlo], v);
-                            keep = true;
-                        } else {
-                            keep = dev::bitmap_set(a.qflag[s.qlo], v);
-                        }
-                        proceed = false;
-                    }
-                }
-            }
-            if (dd && s.pile) {
-                if (a.p.bitmap_frontier)
-                    count_pushes(n, s, false, keep);
-                else
-                    dev::warp_append(a.queue[s.qlo], &n->qcount[s.qlo], a.queue_cap, keep, v, &n->error);
-                if (keep) count_enq(a, acc, false, v);
+                if (pop) dev::bitmap_clear(a.qflag[s.qin], v);  // pop
             }
             // the row offsets are read-only: load them alongside the combine's
             // loads instead of after it (one dependent memory trip less per round)
@@ -1510,7 +1672,7 @@ struct EngineKernel {
                 return;
             }
             const bool heavy = deg > a.p.heavy_threshold;
-            register_heavy(a, s.round & 1u, heavy, v, beg, deg, payload);
+            stage_heavy(a, wlb, s.round & 1u, heavy, v, beg, deg, payload);
             if (heavy) deg = 0;
             expand_warp(app, a, s, wlb, v, beg, deg, payload, dd, acc, lq);
         }
@@ -2037,7 +2199,7 @@ struct EngineKernel {
                 // with neighbouring lanes are combined afterwards.
                 const uint32_t per = (total + 31) / 32;
                 const uint32_t lo = min(total, lane * per), hi = min(total, lo + per);
-                w.partk[0][lane] = w.partk[1][lane] = 0xffffffffu;
+                w.partk(0)[lane] = w.partk(1)[lane] = 0xffffffffu;
                 if (lo < hi) {
                     uint32_t k = owner(w.excl, lo);
                     uint32_t e = lo;
@@ -2067,8 +2229,8 @@ struct EngineKernel {
                             w.pay[k] = r;
                         } else {
                             const int slot = first ? 0 : 1;
-                            w.partk[slot][lane] = k;
-                            w.part[slot][lane] = r;
+                            w.partk(slot)[lane] = k;
+                            w.part(slot)[lane] = r;
                         }
                         first = false;
                         // next destination with edges
@@ -2079,8 +2241,8 @@ struct EngineKernel {
                 {
                     TB r = w.pay[lane];
                     for (uint32_t j = 0; j < 32; ++j) {
-                        if (w.partk[0][j] == lane) r = app.PullReduce(r, w.part[0][j]);
-                        if (w.partk[1][j] == lane) r = app.PullReduce(r, w.part[1][j]);
+                        if (w.partk(0)[j] == lane) r = app.PullReduce(r, w.part(0)[j]);
+                        if (w.partk(1)[j] == lane) r = app.PullReduce(r, w.part(1)[j]);
                     }
                     w.pay[lane] = r;
                 }
@@ -2571,7 +2733,8 @@ struct EngineKernel {
         const unsigned long long now = dev::globaltimer_ns();
         const float round_ms = (float)(now - ps.t_round_start) * 1e-6f;
         ps.vertices_processed += !is_dd(var) ? a.csr.nnodes
-                                 : (a.p.bitmap_frontier && var == V_ASYNC_PUSH_DD) ? dev::ld_l2(&n->popped) : rs.F;
+                                 : ((a.p.bitmap_frontier || rs.pile) && var == V_ASYNC_PUSH_DD) ? dev::ld_l2(&n->popped)
+                                                                                                : rs.F;
         const bool prio_push = a.p.priority && var == V_ASYNC_PUSH_DD;
         const uint32_t out_hi = count_only(a) ? dev::ld_l2(&n->active_count) : qc[rs.qhi];
         const uint32_t out_lo = prio_push ? qc[rs.qlo] : 0;
@@ -2609,22 +2772,20 @@ struct EngineKernel {
             return;
         }
         // rotate worklists
-        uint32_t reset_q;
+        rs.pile = 0;
         if (prio_push && out_hi == 0 && pend == 0) {
-            // near pile drained: open the next priority window over the far pile (driver.cuh:668-675)
+            // near pile drained: open the next priority window over the far pile
+            // (driver.cuh:668-675), whose slot stays where it is
             rs.prio_raw = to_raw<TB>((TB)(from_raw<TB>(rs.prio_raw) + from_raw<TB>(a.p.prio_step_raw)));
-            const uint32_t t = rs.qin;
-            rs.qin = rs.qlo;
-            rs.qlo = t;
-            reset_q = rs.qlo;
             rs.pile = 1;
-        } else {
-            const uint32_t t = rs.qin;
-            rs.qin = rs.qhi;
-            rs.qhi = t;
-            reset_q = rs.qhi;
-            rs.pile = 0;
+            n->qcount[rs.qlo] = 0;
+            n->scout[rs.qlo] = 0;
+            n->heavy_enq[rs.qlo] = 0;
         }
+        const uint32_t consumed = rs.qin;
+        rs.qin = rs.qhi;
+        rs.qhi = consumed;
+        const uint32_t reset_q = rs.qhi;
         n->qcount[reset_q] = 0;
         n->scout[reset_q] = 0;
         n->heavy_enq[reset_q] = 0;
@@ -2646,7 +2807,7 @@ struct EngineKernel {
         rs.variant = next;
         rs.round++;
         rs.F = min(qc[rs.qin], a.queue_cap);
-        rs.heavy_expected = a.p.collect ? he[rs.qin] : (rs.F > 0);
+        rs.heavy_expected = rs.pile ? 1u : a.p.collect ? he[rs.qin] : (rs.F > 0);
         rs.chunks = pend;
         n->middle_count = 0;
         n->pull_chunk_count = 0;
@@ -2734,6 +2895,8 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
     const unsigned long long tmo = a.p.timeout_ns;
     Acc acc;
     acc.reset();
+    acc.stage = nullptr;
+    acc.stage_n = 0;
     PolicyState ps;  // meaningful in block 0 / thread 0 only
     auto nop = [] {};
 
@@ -2763,6 +2926,8 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
     if (!grid_sync(c, tmo, [&] { K::leader_start(a, ps); })) return false;
 
     WarpLB<TB> &my_lb = wlb[dev::warp_id()];
+    if (dev::lane_id() == 0) my_lb.heavy_n = 0;
+    __syncwarp();
     const int lb_push = a.p.lb_push, lb_pull = a.p.lb_pull;
     for (;;) {
         K::load_snap(a, s);
@@ -2778,6 +2943,11 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
             K::sort_emit(a, s);
             if (!grid_sync(c, tmo, nop)) return false;
         }
+        const bool lookahead =
+            var == V_ASYNC_PUSH_DD && a.p.local_depth > 0 && a.p.forced == V_ASYNC_PUSH_DD && reorder_safe(app);
+        acc.stage = var == V_ASYNC_PUSH_DD && !lookahead ? stage : nullptr;  // lookahead fills that memory itself
+        if constexpr (has_take_frontier<App>::value)
+            if (is_dd(var)) app.TakeFrontier(a.queue[s.qin], s.F, K::gthread(), K::nthreads());
         if (s.chunks) {
             // chunks of the heavy vertices the previous push round found (reorder-safe functors only)
             K::heavy_phase(app, a, s, set ^ 1u, true, acc);
@@ -2800,7 +2970,7 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
                     break;
                 }
                 LocalQ *lq = nullptr;
-                if (a.p.local_depth > 0 && a.p.forced == V_ASYNC_PUSH_DD && reorder_safe(app)) {
+                if (lookahead) {
                     if (threadIdx.x == 0) {
                         lq_block.out = 0;
                         lq_block.n[0] = lq_block.n[1] = 0;
