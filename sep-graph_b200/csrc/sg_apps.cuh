@@ -56,6 +56,13 @@ struct BFS : AppBase<TValue, TBuffer, TWeight> {
         return utils::pair<TBuffer, bool>(buf, schedule);
     }
 
+    __forceinline__ __device__ utils::pair<TBuffer, bool> CombinePull(index_t, TValue &value, TBuffer &buffer) const {
+        const bool improved = value > buffer;
+        if (!improved) return utils::pair<TBuffer, bool>(buffer, buffer == kInf);
+        value = buffer;
+        return utils::pair<TBuffer, bool>(buffer + 1, false);
+    }
+
     __forceinline__ __device__ int AccumulateBuffer(index_t, index_t, TBuffer *p_buffer, TBuffer buffer) override {
         TBuffer prev;
         if (m_non_atomic) {
@@ -107,6 +114,11 @@ struct SSSP : AppBase<TValue, TBuffer, TWeight> {
         }
         const bool schedule = this->m_msg_passing == MsgPassing::PUSH ? improved : true;
         return utils::pair<TBuffer, bool>(buf, schedule);
+    }
+
+    __forceinline__ __device__ utils::pair<TBuffer, bool> CombinePull(index_t, TValue &value, TBuffer &buffer) const {
+        if (value > buffer) value = buffer;
+        return utils::pair<TBuffer, bool>(buffer, true);
     }
 
     __forceinline__ __device__ int AccumulateBuffer(index_t, index_t, TWeight weight, TBuffer *p_buffer,
@@ -161,6 +173,18 @@ struct PageRank : AppBase<TValue, TBuffer, TWeight> {
             const index_t deg = this->m_msg_passing == MsgPassing::PUSH
                                     ? this->m_csr_graph.end_edge(node) - this->m_csr_graph.begin_edge(node)
                                     : this->m_csc_graph.out_degree(node);
+            res = (TBuffer)(0.85 * (double)res / (double)deg);
+        }
+        return utils::pair<TBuffer, bool>(res, true);
+    }
+
+    __forceinline__ __device__ utils::pair<TBuffer, bool> CombinePull(index_t node, TValue &value,
+                                                                       TBuffer &buffer) const {
+        TBuffer res = buffer;
+        buffer = (TBuffer)0.0f;
+        const index_t deg = this->m_csc_graph.out_degree(node);
+        if (res > 0) {
+            value += res;
             res = (TBuffer)(0.85 * (double)res / (double)deg);
         }
         return utils::pair<TBuffer, bool>(res, true);
@@ -254,6 +278,14 @@ struct BCForward : AppBase<TValue, TBuffer, TWeight> {
         const bool schedule =
             this->m_msg_passing == MsgPassing::PUSH ? improved : (!improved && *p_buffer == kInf);
         return utils::pair<TBuffer, bool>(buf, schedule);
+    }
+
+    __forceinline__ __device__ utils::pair<TBuffer, bool> CombinePull(index_t node, TValue &value, TBuffer &buffer) const {
+        const bool improved = value > buffer;
+        if (!improved) return utils::pair<TBuffer, bool>(buffer, buffer == kInf);
+        value = buffer;
+        if (this->m_scheduling == common::Scheduling::TOPOLOGY_DRIVEN) m_stack.append(node);
+        return utils::pair<TBuffer, bool>(buffer + 1, false);
     }
 
     __forceinline__ __device__ void add_sigma(index_t dst, unsigned long long s) const {
