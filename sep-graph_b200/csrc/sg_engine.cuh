@@ -211,8 +211,8 @@ inline uint64_t pull_chunk_bound(uint64_t ne) { return ne / kPullChunk + ne / kP
 
 // In-edges per warp tile of the edge-tiled pull: 8 per lane, two 16-byte loads.
 constexpr uint32_t kPullTileEdges = 256;
-// Rows a tile may span (relax tiles) or start (reduce tiles) and still combine
-// them in shared memory first.
+// Row segments of a tile that are combined in shared memory first; a tile with
+// more goes row by row.
 constexpr uint32_t kPullTileRows = 96;
 
 // Leader-only policy state (RunningInfo), lives in block 0 / thread 0.
@@ -238,8 +238,7 @@ struct WarpLB {
             uint32_t beg[32];
             uint32_t src[32];
         };
-        uint32_t rowbeg[kPullTileRows + 1];  // relax tiles: first edges of the tile's rows and of the next one
-        struct {  // reduce tiles: the segments' rows (relative to the tile's first) and sums, marked starts
+        struct {  // edge tiles: the segments' rows (relative to the tile's first) and sums, marked starts
             uint32_t segrow[kPullTileRows];
             TBuffer segsum[kPullTileRows];
             uint32_t mark[8];
@@ -253,8 +252,6 @@ struct WarpLB {
     uint32_t heavy_n, heavy_src[64], heavy_beg[64], heavy_deg[64];
     TBuffer heavy_pay[64];
     uint32_t far_item[64];  // far pile: vertices taken and not processed yet
-    // edge-tiled pull of min-relax functors: per-row minima of one tile
-    TBuffer rowsum[kPullTileRows];
     // bitmap worklist: exclusive scan of the lanes' set bits
     uint32_t scan_excl[32];
 };
@@ -2156,54 +2153,24 @@ struct EngineKernel {
                     offer[j] = c ? dev::ld_l1(offers + src[j]) : none;
                     wt[j] = c && a.csc_w ? dev::ldg_stream(a.csc_w + e0 + j, pol) : 1u;
                 }
-                const uint32_t rlo = __ldg(a.tile_row + t), rhi = __ldg(a.tile_row + t + 1);
-                const bool in_smem = rhi - rlo < kPullTileRows;
-                if (in_smem) {
-                    load_tile_rows(w, crow, rlo, rhi);
-                    for (uint32_t k = lane; k <= rhi - rlo; k += 32) w.rowsum[k] = none;
-                    __syncwarp();
-                }
-                // rows below are relative to rlo
-                auto row_at = [&](uint32_t k, uint32_t e) {
-                    return in_smem ? tile_row_of(w, k, rhi - rlo, e) : row_of(crow, rlo + k, rhi, e) - rlo;
-                };
-                auto row_end = [&](uint32_t k) { return in_smem ? w.rowbeg[k + 1] : __ldg(crow + rlo + k + 1); };
-                auto flush = [&](uint32_t k, TB v) {
-                    if (v == none) return;
-                    if (in_smem) {
-                        atomicMin(&w.rowsum[k], v);
-                    } else if (v < dev::ld_l2(a.buffer + rlo + k)) {
-                        atomicMin(a.buffer + rlo + k, v);
-                        if (dd) mark_pulled(a, s, rlo + k, acc);
-                    }
-                };
-                if (cand) {
-                    uint32_t r = row_at(0, e0);
-                    uint32_t next = row_end(r);
-                    TB run = none;
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const uint32_t e = e0 + j;
-                        if ((cand >> j) & 1u) {
-                            if (e >= next) {
-                                flush(r, run);
-                                run = none;
-                                r = row_at(r + 1, e);
-                                next = row_end(r);
-                            }
-                            const TB x = app.RelaxCandidate(src[j], rlo + r, (TW)wt[j], offer[j]);
-                            run = x < run ? x : run;
-                        }
-                    }
-                    flush(r, run);
-                }
-                if (in_smem) {
-                    __syncwarp();
-                    for (uint32_t k0 = 0; k0 <= rhi - rlo; k0 += 32) {
-                        const uint32_t k = k0 + lane, v = rlo + k;
+                const uint32_t t0 = t * kPullTileEdges, t1 = min(kPullTileEdges, E - t0);
+                const uint32_t rlo = __ldg(a.tile_row + t), rhi = min(__ldg(a.tile_row + t + 1), V - 1);
+                const uint32_t nseg = rank_tile_rows(w, crow, rlo, rhi, t0, t1);
+                auto lower = [](TB x, TB y) { return x < y ? x : y; };
+                if (nseg < kPullTileRows) {
+                    segment_sums(
+                        w, w.segsum, none,
+                        [&](int j, uint32_t k) {
+                            return (cand >> j) & 1u
+                                       ? app.RelaxCandidate(src[j], rlo + w.segrow[k], (TW)wt[j], offer[j])
+                                       : none;
+                        },
+                        lower);
+                    for (uint32_t q0 = 0; q0 < nseg; q0 += 32) {
+                        const uint32_t q = q0 + lane, v = q < nseg ? rlo + w.segrow[q] : rlo;
                         bool want = false;
-                        if (k <= rhi - rlo) {
-                            const TB x = w.rowsum[k];
+                        if (q < nseg) {
+                            const TB x = w.segsum[q];
                             if (x != none && x < dev::ld_l2(a.buffer + v)) {
                                 atomicMin(a.buffer + v, x);
                                 want = dd;
@@ -2216,8 +2183,31 @@ struct EngineKernel {
                         }
                         out.append(want, v);
                     }
-                    __syncwarp();  // rowbeg and rowsum are free for the next tile
+                } else if (cand) {  // a tile of mostly one- and two-edge rows: each lane its own
+                    auto settle = [&](uint32_t r, TB x) {
+                        if (x == none || x >= dev::ld_l2(a.buffer + r)) return;
+                        atomicMin(a.buffer + r, x);
+                        if (dd) mark_pulled(a, s, r, acc);
+                    };
+                    uint32_t r = row_of(crow, rlo, rhi, e0);
+                    uint32_t next = __ldg(crow + r + 1);
+                    TB run = none;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const uint32_t e = e0 + j;
+                        if ((cand >> j) & 1u) {
+                            if (e >= next) {
+                                settle(r, run);
+                                run = none;
+                                r = row_of(crow, r + 1, rhi, e);
+                                next = __ldg(crow + r + 1);
+                            }
+                            run = lower(run, app.RelaxCandidate(src[j], r, (TW)wt[j], offer[j]));
+                        }
+                    }
+                    settle(r, run);
                 }
+                __syncwarp();  // the segments are free for the next tile
             }
             out.flush();
         }
@@ -2338,26 +2328,6 @@ struct EngineKernel {
         return lo;
     }
 
-    // Row starts of a tile's rows [rlo, rhi] (fewer than kPullTileRows) and of
-    // rhi + 1, read together into shared memory: the lanes then search their
-    // rows there, where a search in the row array itself is up to six
-    // dependent L2 loads per lane.
-    static __device__ __forceinline__ void load_tile_rows(WarpLB<TB> &w, const uint32_t *crow, uint32_t rlo,
-                                                          uint32_t rhi) {
-        for (uint32_t k = dev::lane_id(); k <= rhi - rlo + 1; k += 32) w.rowbeg[k] = __ldg(crow + rlo + k);
-    }
-    // Largest k in [lo, hi] with rowbeg[k] <= e.
-    static __device__ __forceinline__ uint32_t tile_row_of(const WarpLB<TB> &w, uint32_t lo, uint32_t hi, uint32_t e) {
-        while (lo < hi) {
-            const uint32_t mid = lo + (hi - lo + 1) / 2;
-            if (w.rowbeg[mid] <= e)
-                lo = mid;
-            else
-                hi = mid - 1;
-        }
-        return lo;
-    }
-
     // tile_row[] of the edge-tiled pull, once per launch (all threads of the team).
     static __device__ void compute_tile_rows(const Args &a) {
         const uint32_t V = a.csc.nnodes, E = a.csc.nedges;
@@ -2398,11 +2368,10 @@ struct EngineKernel {
         return nseg;
     }
 
-    // Sums of the ranked segments of a tile whose edges 8 * lane .. + 7 carry
-    // g[0..7], into sums[].  All 32 lanes call.
-    template <typename T, typename Sum>
-    static __device__ __forceinline__ void segment_sums(const WarpLB<TB> &w, T *sums, const T (&g)[8], T idn,
-                                                        Sum &&sum) {
+    // Sums of the ranked segments of a tile into sums[]; val(j, k) = what this
+    // lane's edge 8 * lane + j adds to its segment k.  All 32 lanes call.
+    template <typename T, typename Val, typename Sum>
+    static __device__ __forceinline__ void segment_sums(const WarpLB<TB> &w, T *sums, T idn, Val &&val, Sum &&sum) {
         const uint32_t lane = dev::lane_id();
         const uint32_t word = w.mark[lane >> 2];
         const uint32_t heads = (word >> ((lane & 3u) * 8u)) & 0xffu;  // rows starting at this lane's edges
@@ -2421,7 +2390,7 @@ struct EngineKernel {
                 run = idn;
                 ++seen;
             }
-            run = sum(run, g[j]);
+            run = sum(run, val(j, k + seen));
         }
         // sum of the open segment up to each lane's end
         bool closed = seen != 0;
@@ -2505,7 +2474,7 @@ struct EngineKernel {
                 const uint32_t rlo = __ldg(a.tile_row + t), rhi = min(__ldg(a.tile_row + t + 1), V - 1);
                 const uint32_t nseg = rank_tile_rows(w, crow, rlo, rhi, t0, t1);
                 if (nseg < kPullTileRows) {
-                    segment_sums(w, segsum, g, 0ull,
+                    segment_sums(w, segsum, 0ull, [&](int j, uint32_t) { return g[j]; },
                                  [&](unsigned long long x, unsigned long long y) { return app.PullSum(x, y); });
                     for (uint32_t q0 = 0; q0 < nseg; q0 += 32) {
                         const uint32_t q = q0 + lane, r = q < nseg ? rlo + w.segrow[q] : rlo;
@@ -2586,7 +2555,8 @@ struct EngineKernel {
                 for (int j = 0; j < 8; ++j) g[j] = e0 + j < E ? dev::ld_l1(vals + s[j]) : idn;
                 const uint32_t nseg = rank_tile_rows(w, crow, rlo, rhi, t0, t1);
                 if (nseg < kPullTileRows) {
-                    segment_sums(w, w.segsum, g, idn, [&](TB x, TB y) { return app.PullReduce(x, y); });
+                    segment_sums(w, w.segsum, idn, [&](int j, uint32_t) { return g[j]; },
+                                 [&](TB x, TB y) { return app.PullReduce(x, y); });
                     for (uint32_t q = lane; q < nseg; q += 32) {
                         const uint32_t r = rlo + w.segrow[q];
                         accumulate<App, TB, TW>(app, a.csc_w, r, r, 0, a.buffer + r, w.segsum[q]);
