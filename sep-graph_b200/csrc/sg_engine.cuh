@@ -542,7 +542,9 @@ __device__ __forceinline__ bool grid_sync(Ctrl *c, unsigned long long timeout_ns
     return s_ok != 0;
 }
 
-template <typename App, typename TV, typename TB, typename TW>
+// kCollect = false: no policy statistics are kept (kernels of one forced
+// variant, which runs that trace their rounds do not take).
+template <typename App, typename TV, typename TB, typename TW, bool kCollect = true>
 struct EngineKernel {
     using Args = KArgs<TV, TB, TW>;
     using Snap = RoundState;
@@ -561,7 +563,7 @@ struct EngineKernel {
     // needed and the two dependent loads are skipped (the round then always
     // runs its chunk phase).
     static __device__ __forceinline__ void count_enq(const Args &a, Acc &acc, bool hi, uint32_t v) {
-        if (a.p.collect || may_be_dense(a)) acc.count(hi, out_degree(a, v), a.p.heavy_threshold);
+        if ((kCollect && a.p.collect) || may_be_dense(a)) acc.count(hi, out_degree(a, v), a.p.heavy_threshold);
     }
 
     // Dense push rounds.  With most of the edges in the worklist, nearly every
@@ -621,10 +623,15 @@ struct EngineKernel {
         if (acc.stage) flush_stage(a, acc, q_hi);
         const unsigned long long wide[3] = {acc.scout_hi, acc.scout_lo, acc.edges};
         const uint32_t narrow[6] = {acc.heavy_hi, acc.heavy_lo, acc.active, acc.push_hi, acc.push_lo, acc.popped};
+        bool some = false;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) some |= wide[k] != 0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) some |= narrow[k] != 0;
+        if (!__syncthreads_or(some)) return;  // the small rounds' common case: nothing in the whole block
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            unsigned long long x = 0;
-            if (__any_sync(dev::kFullMask, wide[k] != 0)) x = dev::warp_sum(wide[k]);
+            const unsigned long long x = dev::warp_sum(wide[k]);
             if (dev::lane_id() == 0) part[dev::warp_id()][k] = x;
         }
 #pragma unroll
@@ -1763,12 +1770,14 @@ struct EngineKernel {
             // chain of L2 or HBM trips (BFS on symmetric RMAT-23: 167 and 205 us
             // for the 8.4 M vertices of a round)
             constexpr int kStep = 4;
+            const bool several = (uint64_t)nwarps() * 32 < N;  // else a warp has one word at most
             for (uint64_t w0 = gwarp(); w0 * 32 < N; w0 += (uint64_t)kStep * nwarps()) {
                 TV val[kStep], val0[kStep];
                 TB buf[kStep], buf0[kStep];
                 bool want[kStep];
 #pragma unroll
                 for (int k = 0; k < kStep; ++k) {
+                    if (k > 0 && !several) break;
                     const uint64_t v = (w0 + (uint64_t)k * nwarps()) * 32 + lane;
                     if (v < N) {
                         val0[k] = dev::ld_l2(a.value + v);
@@ -1777,8 +1786,9 @@ struct EngineKernel {
                 }
 #pragma unroll
                 for (int k = 0; k < kStep; ++k) {
-                    const uint64_t v = (w0 + (uint64_t)k * nwarps()) * 32 + lane;
                     want[k] = false;
+                    if (k > 0 && !several) continue;
+                    const uint64_t v = (w0 + (uint64_t)k * nwarps()) * 32 + lane;
                     if (v >= N) continue;
                     val[k] = val0[k];
                     buf[k] = buf0[k];
@@ -1804,6 +1814,7 @@ struct EngineKernel {
                 }
 #pragma unroll
                 for (int k = 0; k < kStep; ++k) {
+                    if (k > 0 && !several) break;
                     const uint64_t w = w0 + (uint64_t)k * nwarps();
                     const uint64_t v = w * 32 + lane;
                     if (split && want[k]) list_pull_chunks(a, (uint32_t)v, beg[k], end[k] - beg[k], acc);
@@ -2926,7 +2937,7 @@ struct EngineKernel {
 // other variants' code, registers and shared memory then fall away.
 template <typename App, typename TV, typename TB, typename TW, int kForced = -1>
 __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
-    using K = EngineKernel<App, TV, TB, TW>;
+    using K = EngineKernel<App, TV, TB, TW, (kForced < 0)>;
     __shared__ RoundState s;
     __shared__ WarpLB<TB> wlb[kWarpsPerBlock];
     __shared__ LocalQ lq_block;

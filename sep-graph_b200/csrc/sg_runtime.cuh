@@ -526,12 +526,12 @@ sg_status run_engine(sg_graph *g, App app, const EngineConfig &cfg, TV *value, T
     static std::atomic<int> occupancy[3] = {{0}, {0}, {0}};  // per template instantiation: all variants, push, pull
     int which = 0;
     if constexpr (specialised<App, TB, TW>(V_ASYNC_PUSH_DD))
-        if (cfg.forced == V_ASYNC_PUSH_DD) {
+        if (cfg.forced == V_ASYNC_PUSH_DD && !cfg.trace) {
             kernel = (const void *)hybrid_engine_kernel<App, TV, TB, TW, V_ASYNC_PUSH_DD>;
             which = 1;
         }
     if constexpr (specialised<App, TB, TW>(V_SYNC_PULL_TD))
-        if (cfg.forced == V_SYNC_PULL_TD) {
+        if (cfg.forced == V_SYNC_PULL_TD && !cfg.trace) {
             kernel = (const void *)hybrid_engine_kernel<App, TV, TB, TW, V_SYNC_PULL_TD>;
             which = 2;
         }
