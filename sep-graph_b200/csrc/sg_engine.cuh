@@ -99,10 +99,16 @@ struct Counters {
     uint32_t pull_chunk_count;  // entries of KArgs::pull_chunks in the current pull round
 };
 
+// The barrier's words, the round snapshot and the counters have 128-byte lines
+// of their own: the waiting blocks poll bar_gen, and the round's atomics and the
+// arrivals on its line queued behind those reads (64 BFS on symmetric RMAT-22
+// 5.2 -> 4.5 ms).
 struct Ctrl {
-    uint32_t bar_count, bar_gen, pad0, pad1;
-    RoundState rs;
-    Counters cnt;
+    uint32_t bar_count;
+    alignas(128) uint32_t bar_gen;
+    uint32_t pad0;
+    alignas(128) RoundState rs;
+    alignas(128) Counters cnt;
     // results, written by the leader when the loop ends
     uint32_t round, max_iteration_reached, n_trace, error;
     uint32_t rounds_by_variant[8];
@@ -3126,17 +3132,19 @@ constexpr bool specialised(int v) {
 }
 
 // Resident blocks per SM that the kernels are compiled for (registers): the
-// unweighted functors' rounds fit 51 registers, relaxation with eight edges in
-// flight per lane takes 80 (at 64, four blocks, it spills: 256 SSSP in one call
-// 50.5 -> 55.8 ms).
-template <typename TW>
+// unweighted functors' rounds fit 51 registers, push PageRank with the tiles of
+// its dense rounds takes 64 (1,000,003 vertices 15.9 -> 14.6 ms), relaxation with
+// eight edges in flight per lane 80 (at 64, four blocks, it spills: 256 SSSP in
+// one call 50.5 -> 55.8 ms).
+template <typename TW, int kForced>
 constexpr int min_blocks() {
-    return std::is_same<TW, graphs::NoWeight>::value ? 5 : 3;
+    return !std::is_same<TW, graphs::NoWeight>::value ? 3 : kForced == V_ASYNC_PUSH_DD ? 4 : 5;
 }
 
 // One query: the whole cooperative grid is the team.
 template <typename App, typename TV, typename TB, typename TW, int kForced = -1>
-__global__ void __launch_bounds__(kBlockThreads, min_blocks<TW>()) hybrid_engine_kernel(const App app_in, KArgs<TV, TB, TW> a) {
+__global__ void __launch_bounds__(kBlockThreads, min_blocks<TW, kForced>())
+    hybrid_engine_kernel(const App app_in, KArgs<TV, TB, TW> a) {
     set_team(blockIdx.x, gridDim.x, a.ctrl);
     run_instance<App, TV, TB, TW, kForced>(app_in, a);
 }
@@ -3196,7 +3204,7 @@ __device__ __forceinline__ void write_result(BatchResult *r, const Ctrl *c, uint
 // and state never leave the device; the batch is one launch (capturable in a
 // CUDA graph).
 template <typename App, typename TV, typename TB, typename TW, int kForced = -1>
-__global__ void __launch_bounds__(kBlockThreads, min_blocks<TW>() < 4 ? min_blocks<TW>() : 4)
+__global__ void __launch_bounds__(kBlockThreads, min_blocks<TW, kForced>() < 4 ? min_blocks<TW, kForced>() : 4)
     batched_engine_kernel(const BatchQuery<App, TV> *queries, uint32_t nq, const TeamSpace<TB> *spaces,
                           uint32_t team_blocks, uint32_t *next_query, BatchResult *results, Params p) {
     const uint32_t team = blockIdx.x / team_blocks;
