@@ -266,9 +266,13 @@ __global__ void __launch_bounds__(kMbThreads) msbc_kernel(MbArgs a) {
                 deg = __ldg(a.crow + v + 1) - b;
                 if (deg <= kMbThreadDeg) want = a.full & ~__ldcg(a.seen + v);
                 if (want) {
-                    for (uint32_t e = b; e < b + deg; ++e) {
-                        nm |= __ldcg(a.fr + __ldg(a.ccol + e));
-                        if ((nm & want) == want) break;
+                    for (uint32_t e = b; e < b + deg && (nm & want) != want; e += 4) {  // four masks in flight
+                        uint32_t u[4], f[4];
+#pragma unroll
+                        for (uint32_t t = 0; t < 4; ++t) u[t] = __ldg(a.ccol + min(e + t, b + deg - 1));
+#pragma unroll
+                        for (uint32_t t = 0; t < 4; ++t) f[t] = __ldcg(a.fr + u[t]);
+                        nm |= f[0] | f[1] | f[2] | f[3];
                     }
                     nm &= want;
                 }
