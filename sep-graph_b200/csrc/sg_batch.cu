@@ -1003,7 +1003,7 @@ sg_status prepare_batch(sg_ctx *ctx, sgb::Workspace &ws, std::vector<engine::Bat
     sg_status st;
     if ((st = ws_get(ctx, ws, "b_buf", T * nv_max, &buf)) != SG_OK) return st;
     if ((st = ws_get(ctx, ws, "b_tmp", T * nv_max, &tmp)) != SG_OK) return st;
-    if ((st = ws_get(ctx, ws, "b_q", T * 3 * nv_max, &qq)) != SG_OK) return st;
+    if ((st = ws_get(ctx, ws, "b_q", T * 2 * nv_max, &qq)) != SG_OK) return st;
     if ((st = ws_get(ctx, ws, "b_bm", T * 2 * nwords, &bm)) != SG_OK) return st;
     if ((st = ws_get(ctx, ws, "b_fl", T * 3 * nwords, &fl)) != SG_OK) return st;
     if ((st = ws_get(ctx, ws, "b_mid", T * nv_max, &mid)) != SG_OK) return st;
@@ -1025,7 +1025,7 @@ sg_status prepare_batch(sg_ctx *ctx, sgb::Workspace &ws, std::vector<engine::Bat
         s.buffer = buf + t * nv_max;
         s.tmp = tmp + t * nv_max;
         for (int k = 0; k < 3; ++k) {
-            s.queue[k] = qq + (t * 3 + k) * nv_max;
+            s.queue[k] = k < 2 ? qq + (t * 2 + k) * nv_max : nullptr;
             s.qflag[k] = fl + (t * 3 + k) * nwords;
         }
         s.bitmap[0] = bm + (t * 2) * nwords;

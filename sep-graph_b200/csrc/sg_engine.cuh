@@ -99,15 +99,15 @@ struct Counters {
     uint32_t pull_chunk_count;  // entries of KArgs::pull_chunks in the current pull round
 };
 
-// The barrier's words, the round snapshot and the counters have 128-byte lines
-// of their own: the waiting blocks poll bar_gen, and the round's atomics and the
-// arrivals on its line queued behind those reads (64 BFS on symmetric RMAT-22
-// 5.2 -> 4.5 ms).
+// The barrier's words and the round snapshot share one 128-byte line (a release
+// that has to reach several lines took half a microsecond longer per barrier);
+// the counters have lines of their own: the waiting blocks poll bar_gen, and the
+// round's atomics on its line queued behind those reads (64 BFS on symmetric
+// RMAT-22 5.2 -> 4.5 ms).
 struct Ctrl {
-    uint32_t bar_count;
-    alignas(128) uint32_t bar_gen;
-    uint32_t pad0;
-    alignas(128) RoundState rs;
+    alignas(128) uint32_t bar_count;
+    uint32_t bar_gen, pad0, pad1;
+    RoundState rs;
     alignas(128) Counters cnt;
     // results, written by the leader when the loop ends
     uint32_t round, max_iteration_reached, n_trace, error;
@@ -175,7 +175,7 @@ struct KArgs {
     TValue *value;
     TBuffer *buffer;
     TBuffer *tmp;
-    uint32_t *queue[3];
+    uint32_t *queue[3];  // worklists; slot 2, the far pile, is its queued bitmap alone (null)
     uint32_t queue_cap;
     uint32_t *bitmap[2];
     uint32_t *qflag[3];  // queued bitmap of each worklist slot

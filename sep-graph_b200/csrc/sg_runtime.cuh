@@ -472,7 +472,6 @@ sg_status run_engine(sg_graph *g, App app, const EngineConfig &cfg, TV *value, T
     SG_TRY_CUDA(ctx, ws.get("tmp", nv, &a.tmp));
     SG_TRY_CUDA(ctx, ws.get("q0", nv, &a.queue[0]));
     SG_TRY_CUDA(ctx, ws.get("q1", nv, &a.queue[1]));
-    SG_TRY_CUDA(ctx, ws.get("q2", nv, &a.queue[2]));
     SG_TRY_CUDA(ctx, ws.get("bm0", nwords, &a.bitmap[0]));
     SG_TRY_CUDA(ctx, ws.get("bm1", nwords, &a.bitmap[1]));
     SG_TRY_CUDA(ctx, ws.get("fl0", nwords, &a.qflag[0]));
