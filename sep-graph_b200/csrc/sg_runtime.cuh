@@ -387,7 +387,11 @@ inline int resident_blocks_per_sm(const sg_ctx *ctx, int max_bps) {
 // the per-level barrier (fewer blocks), large dense ones by memory latency
 // (more).  Measured on B200: 16 BFS on the 4096^2 grid 197 / 229 / 288 ms with
 // 2 / 4 / 6 blocks; 64 BFS and 32 BC on symmetric RMAT-22 9.4 -> 8.2 and
-// 23.3 -> 21.1 ms from 4 to 6; RMAT-16 best with 4.  On a sparse graph a
+// 23.3 -> 21.1 ms from 4 to 6.  With 2 / 3 / 4 / 5 / 6 blocks, 32 BC on R-MAT
+// graphs of 20,011 vertices (0.5 M edges) 0.76 / 0.77 / 0.91 / 1.01 / 1.02 ms, of
+// 100,003 (2.8 M) 1.49 / 1.29 / 1.16 / 1.31 / 1.29, of 700,001 (20 M) 7.7 / 5.9 /
+// 5.3 / 4.9 / 4.9, and 64 BFS 0.21 / 0.22 / 0.24 / 0.26 / 0.26, 0.34 / 0.32 / 0.33 /
+// 0.35 / 0.35, 1.38 / 1.11 / 0.99 / 0.93 / 0.93.  On a sparse graph a
 // round's work grows with the sources times the wavefront (about sqrt(V) on
 // a grid), and a large one fills more blocks: push-only multi-source BFS, 64
 // sources on the 4096^2 grid 1030 / 650 / 521 / 462 ms with 1 / 2 / 3 / 4
@@ -396,7 +400,8 @@ inline int resident_blocks_per_sm(const sg_ctx *ctx, int max_bps) {
 inline int ms_blocks_per_sm(uint32_t nv, uint64_t ne, uint32_t nsrc) {
     const double avg_deg = nv ? (double)ne / nv : 0.0;
     if (avg_deg < 8) return (double)nsrc * std::sqrt((double)nv) >= 131072.0 ? 4 : 2;
-    return ne >= (1ull << 25) ? 6 : 4;
+    if (ne < (1ull << 20)) return 2;
+    return ne >= (1ull << 23) ? 6 : 4;
 }
 
 // Resident blocks per SM when the caller does not choose: small graphs are
