@@ -106,7 +106,8 @@ typedef struct sg_options {
                                  output slot's bitmap itself (fire-and-forget bit sets, no appends) */
     int32_t l2_persist;       /* L2 persistence window on the array a launch updates at random (the tentative
                                  values; the pulled values of a topology-driven pull) for single-query
-                                 calls: 0 = library choice (on where the device supports it), 1 = on,
+                                 calls: 0 = library choice (on where the device supports it and the
+                                 array has 4 MB or more), 1 = on,
                                  -1 = off.  Set on the launch's stream for that launch only; the L2
                                  set-aside it needs is returned when the last context of the device is
                                  destroyed. */
