@@ -495,7 +495,6 @@ __global__ void __launch_bounds__(kMsThreads) msbfs_fused_kernel(MsArgs a) {
     };
     if (!engine::grid_sync(c, a.timeout_ns, start)) return;
 
-    __shared__ uint32_t stage[kMsThreads / 32][256];
     uint32_t u4[4];
     for (;;) {
         if (threadIdx.x < 4)
@@ -505,7 +504,6 @@ __global__ void __launch_bounds__(kMsThreads) msbfs_fused_kernel(MsArgs a) {
         const uint32_t p = s.qin, q = p ^ 1u;
         const bool expand = s.pile == 0;
         const uint32_t *T = a.active[p];
-        dev::WarpStage out(stage[dev::warp_id()], 256, a.active[q], &n->qcount[q], a.nv, &n->error);
         unsigned long long edges = 0;
         // OR f into up to four neighbours col[e + k * stride] (e + k * stride < end)
         // of next[q]; returns the bits k whose OR was that vertex's first (it is
@@ -559,7 +557,7 @@ __global__ void __launch_bounds__(kMsThreads) msbfs_fused_kernel(MsArgs a) {
             const uint32_t steps = __reduce_max_sync(dev::kFullMask, (mine + 3u) >> 2);
             for (uint32_t st = 0; st < steps; ++st) {
                 const uint32_t first = push4(beg + 4 * st, beg + mine, 1, nb);
-                out.append4(first, u4);
+                dev::warp_append4(a.active[q], &n->qcount[q], a.nv, first, u4, &n->error);
             }
             edges += mine;
             // larger lists: a whole warp per vertex
@@ -571,12 +569,11 @@ __global__ void __launch_bounds__(kMsThreads) msbfs_fused_kernel(MsArgs a) {
                 const unsigned long long fj = __shfl_sync(dev::kFullMask, nb, j);
                 for (uint32_t off = 0; off < dj; off += 128) {
                     const uint32_t first = push4(bj + off + lane, bj + dj, 32, fj);
-                    out.append4(first, u4);
+                    dev::warp_append4(a.active[q], &n->qcount[q], a.nv, first, u4, &n->error);
                 }
                 if (lane == 0) edges += dj;
             }
         }
-        out.flush();
         edges = dev::warp_sum(edges);
         if (lane == 0 && edges) atomicAdd(&n->edges_processed, edges);
         auto end_round = [&] {

@@ -1,5 +1,5 @@
 // Device primitives of the B200 hybrid engine: a bounded grid barrier whose
-// last arriving block runs a single-thread callback, warp-aggregated worklist
+// last arriving block runs a single-thread callback, staged worklist
 // appends, bitmap frontier helpers and small warp collectives.
 //
 // Reference counterparts: cub::GridBarrier (unbounded spin, used by the fused
@@ -165,28 +165,6 @@ __device__ __forceinline__ T warp_sum(T x) {
     return x;
 }
 
-// Warp-aggregated append: one atomicAdd per warp, items packed in lane order.
-// Must be called by all 32 lanes.  A reservation past `cap` writes nothing and
-// raises kErrCapacity instead of the reference's silent out-of-bounds write
-// (queue.cuh:86 asserts only in debug builds).
-__device__ __forceinline__ uint32_t warp_append(uint32_t *queue, uint32_t *count, uint32_t cap, bool want,
-                                                uint32_t item, uint32_t *err) {
-    const uint32_t m = __ballot_sync(kFullMask, want);
-    if (m == 0) return 0;
-    const uint32_t leader = __ffs(m) - 1;
-    uint32_t base = 0;
-    if (lane_id() == leader) base = atomicAdd(count, (uint32_t)__popc(m));
-    base = __shfl_sync(kFullMask, base, leader);
-    if (want) {
-        const uint32_t pos = base + __popc(m & lanemask_lt());
-        if (pos < cap)
-            queue[pos] = item;
-        else
-            atomicOr(err, kErrCapacity);
-    }
-    return m;
-}
-
 // A warp's worklist appends of a dense phase, collected in `cap` (> 32) words
 // of shared memory and moved to the worklist with one reservation per nearly
 // `cap` items: the counter is a single word, and one returning atomic per 32
@@ -242,6 +220,34 @@ struct WarpStage {
     }
 };
 
+// Appends, for every lane, items[k] for each set bit k (< 4) of `which`, with
+// one atomic per warp on `count`; all 32 lanes must call it.
+__device__ __forceinline__ void warp_append4(uint32_t *queue, uint32_t *count, uint32_t cap, uint32_t which,
+                                             const uint32_t (&items)[4], uint32_t *err) {
+    const uint32_t c = __popc(which);
+    uint32_t incl = c;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFullMask, incl, d);
+        if (lane_id() >= (uint32_t)d) incl += y;
+    }
+    const uint32_t total = __shfl_sync(kFullMask, incl, 31);
+    if (total == 0) return;
+    uint32_t base = 0;
+    if (lane_id() == 31) base = atomicAdd(count, total);
+    base = __shfl_sync(kFullMask, base, 31);
+    uint32_t pos = base + incl - c;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if ((which >> k) & 1u) {
+            if (pos < cap)
+                queue[pos] = items[k];
+            else
+                atomicOr(err, kErrCapacity);
+            ++pos;
+        }
+}
+
 __device__ __forceinline__ bool bitmap_test(const uint32_t *bm, uint32_t v) {
     return (ld_l2(bm + (v >> 5)) >> (v & 31u)) & 1u;
 }
@@ -265,9 +271,6 @@ __device__ __forceinline__ void bitmap_and_nr(uint32_t *word, uint32_t bits) {
 }
 __device__ __forceinline__ void bitmap_or_nr(uint32_t *word, uint32_t bits) {
     asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" ::"l"(word), "r"(bits) : "memory");
-}
-__device__ __forceinline__ void red_add(uint32_t *p, uint32_t v) {
-    asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
 // Bounded grid barrier for a cooperative launch (all blocks co-resident).
