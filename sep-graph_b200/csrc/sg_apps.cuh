@@ -254,7 +254,8 @@ struct BCForward : AppBase<TValue, TBuffer, TWeight> {
     unsigned long long *m_sigmas;
     uint32_t *m_p_search_depth;
     LevelStack m_stack;
-    uint32_t m_taken = 0;  // vertices TakeFrontier appended this round
+    bool m_frontier_taken = false;  // set by the engine: this round began with TakeFrontier
+    uint32_t m_taken = 0;           // vertices it appended
 
     BCForward(index_t source, unsigned long long *sigmas, uint32_t *search_depth, LevelStack stack)
         : m_source_node(source), m_sigmas(sigmas), m_p_search_depth(search_depth), m_stack(stack) {}
@@ -272,8 +273,7 @@ struct BCForward : AppBase<TValue, TBuffer, TWeight> {
         if (improved) {
             *p_value = buf;
             buf += 1;
-            // data-driven rounds: TakeFrontier has it
-            if (this->m_scheduling == common::Scheduling::TOPOLOGY_DRIVEN) m_stack.append(node);
+            if (!m_frontier_taken) m_stack.append(node);
         }
         const bool schedule =
             this->m_msg_passing == MsgPassing::PUSH ? improved : (!improved && *p_buffer == kInf);
@@ -284,7 +284,7 @@ struct BCForward : AppBase<TValue, TBuffer, TWeight> {
         const bool improved = value > buffer;
         if (!improved) return utils::pair<TBuffer, bool>(buffer, buffer == kInf);
         value = buffer;
-        if (this->m_scheduling == common::Scheduling::TOPOLOGY_DRIVEN) m_stack.append(node);
+        if (!m_frontier_taken) m_stack.append(node);
         return utils::pair<TBuffer, bool>(buffer + 1, false);
     }
 
@@ -327,9 +327,10 @@ struct BCForward : AppBase<TValue, TBuffer, TWeight> {
         return buffer < prev ? this->ACCUMULATE_SUCCESS_CONTINUE : this->ACCUMULATE_FAILURE_CONTINUE;
     }
 
-    // A level-synchronous round's worklist is exactly the vertices whose level
-    // its combines fix, so the stack segment is a copy of it; appending from the
-    // combines was one reservation per 32 vertices on one counter.
+    // A level-synchronous round's queue is exactly the vertices whose level its
+    // combines fix, so the stack segment is a copy of it; appending from the
+    // combines is one reservation per 32 vertices on one counter.  Rounds without
+    // such a queue (topology-driven, bitmap worklists) append from the combines.
     __forceinline__ __device__ void TakeFrontier(const uint32_t *items, uint32_t n, uint32_t thread, uint32_t nthreads) {
         const uint32_t base = dev::ld_l2(m_stack.count);  // PostComputation adds n
         for (uint32_t i = thread; i < n; i += nthreads) {
@@ -343,8 +344,7 @@ struct BCForward : AppBase<TValue, TBuffer, TWeight> {
 
     __forceinline__ __device__ bool IsActiveNode(index_t, TBuffer buffer) const override { return buffer != kInf; }
     __forceinline__ __device__ void PostComputation() override {
-        m_stack.push(m_taken);
-        m_taken = 0;
+        m_stack.push(m_frontier_taken ? m_taken : 0u);
     }
 };
 

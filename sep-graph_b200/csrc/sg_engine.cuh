@@ -423,10 +423,13 @@ constexpr uint32_t kDenseShare = 2;
 constexpr uint32_t kTermShare = 3;
 
 // Optional functor extension (no reference counterpart): a functor that keeps
-// the vertices of every data-driven round declares
+// the vertices of every round declares
 //   __device__ void TakeFrontier(const index_t *items, uint32_t n, uint32_t thread, uint32_t nthreads)
-// called by all threads of the team before the round's combines with its input
-// worklist (each vertex once; thread = 0 .. nthreads - 1).
+//   bool m_frontier_taken
+// In rounds whose input worklist is a queue, all threads of the team call
+// TakeFrontier with it before the combines (each vertex once; thread = 0 ..
+// nthreads - 1) and m_frontier_taken is true; in the others (topology-driven,
+// bitmap worklists, the far pile) it is false and the combines see the vertices.
 template <typename App, typename = void>
 struct has_take_frontier : std::false_type {};
 template <typename App>
@@ -3026,8 +3029,10 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
         const bool lookahead =
             var == V_ASYNC_PUSH_DD && a.p.local_depth > 0 && a.p.forced == V_ASYNC_PUSH_DD && reorder_safe(app);
         acc.stage = var == V_ASYNC_PUSH_DD && !lookahead ? stage : nullptr;  // lookahead fills that memory itself
-        if constexpr (has_take_frontier<App>::value)
-            if (is_dd(var)) app.TakeFrontier(a.queue[s.qin], s.F, K::gthread(), K::nthreads());
+        if constexpr (has_take_frontier<App>::value) {
+            app.m_frontier_taken = is_dd(var) && !a.p.bitmap_frontier && !s.pile;
+            if (app.m_frontier_taken) app.TakeFrontier(a.queue[s.qin], s.F, K::gthread(), K::nthreads());
+        }
         if (s.chunks) {
             // chunks of the heavy vertices the previous push round found (reorder-safe functors only)
             K::heavy_phase(app, a, s, set ^ 1u, true, acc);

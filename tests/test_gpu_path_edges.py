@@ -75,6 +75,24 @@ def test_bc_hub(ctx, k, variant, back):
     G.close()
 
 
+@pytest.mark.parametrize("k", [1, 33, 513, 5000])
+@pytest.mark.parametrize("opts", [{"worklist": 2}, {"worklist": 1}, {"wl_sort": True}])
+def test_bc_level_stack_by_worklist(ctx, k, opts):
+    """Path counts and dependencies do not depend on how the rounds keep their worklists."""
+    nv, s, d = _hub(k)
+    off, idx, _ = _csr(nv, np.concatenate([s, d]), np.concatenate([d, s]))
+    G = ctx.graph_from_csr(off, idx)
+    queries = [(G, 0), (G, nv - 1), (G, 1)]
+    out = ctx.bc_batch(queries, variant="async_push_dd", lb_push="fine", **opts)[0]
+    for q, (_, src) in enumerate(queries):
+        want, sig, _ = oracle.bc_f64(off, idx, src)
+        bc, sigma, _ = G.bc(src, variant="async_push_dd", lb_push="fine", **opts)
+        assert np.array_equal(sigma.astype(np.float64), sig)
+        assert np.all(np.abs(bc - want) <= 1e-4 * np.abs(want) + 1e-5)
+        assert np.all(np.abs(out[q] - want) <= 1e-4 * np.abs(want) + 1e-5)
+    G.close()
+
+
 def _random(nv, m, seed, lo=0):
     r = np.random.default_rng(seed)
     return r.integers(lo, nv, m).astype(np.uint32), r.integers(lo, nv, m).astype(np.uint32)
