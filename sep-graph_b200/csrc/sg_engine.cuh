@@ -2182,7 +2182,7 @@ struct EngineKernel {
                     wt[j] = c && a.csc_w ? dev::ldg_stream(a.csc_w + e0 + j, pol) : 1u;
                 }
                 const uint32_t t0 = t * kPullTileEdges, t1 = min(kPullTileEdges, E - t0);
-                const uint32_t rlo = __ldg(a.tile_row + t), rhi = min(__ldg(a.tile_row + t + 1), V - 1);
+                const uint32_t rlo = dev::ld_l1(a.tile_row + t), rhi = min(dev::ld_l1(a.tile_row + t + 1), V - 1);
                 const uint32_t nseg = rank_tile_rows(w, crow, rlo, rhi, t0, t1);
                 auto lower = [](TB x, TB y) { return x < y ? x : y; };
                 if (nseg < kPullTileRows) {
@@ -2356,7 +2356,9 @@ struct EngineKernel {
         return lo;
     }
 
-    // tile_row[] of the edge-tiled pull, once per launch (all threads of the team).
+    // tile_row[] of the edge-tiled pull, once per query (all threads of the team).
+    // A batched launch rewrites it for every query a team claims, so it is read
+    // with ordinary loads after the barrier (ld_l1), not as read-only data.
     static __device__ void compute_tile_rows(const Args &a) {
         const uint32_t V = a.csc.nnodes, E = a.csc.nedges;
         const uint32_t T = (E + kPullTileEdges - 1) / kPullTileEdges;
@@ -2499,7 +2501,7 @@ struct EngineKernel {
                     offer = dev::ld_l2(offers + __shfl_sync(dev::kFullMask, u, __ffs(any) - 1));
                     have_offer = true;
                 }
-                const uint32_t rlo = __ldg(a.tile_row + t), rhi = min(__ldg(a.tile_row + t + 1), V - 1);
+                const uint32_t rlo = dev::ld_l1(a.tile_row + t), rhi = min(dev::ld_l1(a.tile_row + t + 1), V - 1);
                 const uint32_t nseg = rank_tile_rows(w, crow, rlo, rhi, t0, t1);
                 if (nseg < kPullTileRows) {
                     segment_sums(w, segsum, 0ull, [&](int j, uint32_t) { return g[j]; },
@@ -2567,7 +2569,7 @@ struct EngineKernel {
             for (uint32_t t = gwarp(); t < T; t += nwarps()) {
                 const uint32_t t0 = t * kPullTileEdges, t1 = min(kPullTileEdges, E - t0);  // first edge, edges
                 const uint32_t e0 = t0 + lane * 8u;
-                const uint32_t rlo = __ldg(a.tile_row + t), rhi = min(__ldg(a.tile_row + t + 1), V - 1);
+                const uint32_t rlo = dev::ld_l1(a.tile_row + t), rhi = min(dev::ld_l1(a.tile_row + t + 1), V - 1);
                 // Lane l gathers edges l, l + 32, ..: a row's sources ascend, so
                 // neighbouring lanes share lines in its dense stretches; the
                 // values then change lanes through shared memory.  PageRank on

@@ -117,6 +117,35 @@ def test_sssp_relax_tiles(ctx, nv, m, variant):
     G.close()
 
 
+@pytest.mark.parametrize("algo", ["sssp", "bc"])
+@pytest.mark.parametrize("variant", ["async_pull_dd", "auto"])
+def test_batch_teams_take_graphs_in_turn(ctx, algo, variant):
+    """Far more queries than teams, over graphs whose tiles hold different rows: a team's tile rows are
+    rewritten for each query it claims."""
+    graphs, wants = [], []
+    for k, (nv, m) in enumerate([(3000, 40000), (40, 9000), (20000, 41000), (700, 20001)]):
+        s, d = _random(nv, m, 17 * k + nv)
+        if algo == "sssp":
+            off, idx, w = _csr(nv, s, d, np.random.default_rng(k).integers(1, 1000, m).astype(np.uint32))
+            graphs.append(ctx.graph_from_csr(off, idx, w))
+            wants.append([oracle.sssp(off, idx, w, src) for src in range(3)])
+        else:
+            off, idx, _ = _csr(nv, s, d)
+            graphs.append(ctx.graph_from_csr(off, idx))
+            wants.append([oracle.bc_f64(off, idx, src)[0] for src in range(3)])
+    picks = [(q % 4, (q // 4) % 3) for q in range(600)]
+    call = ctx.sssp_batch if algo == "sssp" else ctx.bc_batch
+    outs = call([(graphs[g], src) for g, src in picks], team_blocks=4, blocks_per_sm=1, variant=variant,
+                max_iteration=100000)[0]
+    for (g, src), out in zip(picks, outs):
+        if algo == "sssp":
+            assert np.array_equal(out, wants[g][src])
+        else:
+            assert np.all(np.abs(out - wants[g][src]) <= 1e-4 * np.abs(wants[g][src]) + 1e-5)
+    for G in graphs:
+        G.close()
+
+
 @pytest.mark.parametrize("nv,m", TILES + [(20000, 320000)])
 @pytest.mark.parametrize("variant", ["sync_pull_td", "async_push_dd", "auto"])
 @pytest.mark.parametrize("no_csc", [False, True])
