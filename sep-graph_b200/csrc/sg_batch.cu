@@ -121,7 +121,10 @@ struct MsLeader {
 __device__ __forceinline__ uint32_t gthread() { return blockIdx.x * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ uint32_t nthreads() { return gridDim.x * blockDim.x; }
 
-__global__ void __launch_bounds__(kMsThreads) msbfs_kernel(MsArgs a) {
+// Five blocks per SM: the gathers wait on L2, and at the 64 registers the
+// compiler takes without the bound only four fit (symmetric RMAT-22, 64 sources,
+// 5.4 ms against 4.9).
+__global__ void __launch_bounds__(kMsThreads, 5) msbfs_kernel(MsArgs a) {
     Ctrl *c = a.ctrl;
     engine::set_team(blockIdx.x, gridDim.x, c);
     __shared__ engine::RoundState s;
