@@ -754,7 +754,19 @@ __global__ void row_lengths_kernel(const uint32_t *row_begin, const uint32_t *ro
 
 // Source of every CSR entry.  A block takes 4096 entries, finds the rows they
 // span with two searches, writes each non-empty row at its first entry in
-// shared memory and spreads it with a running maximum.
+// shared memory and spreads it with a running maximum.  Entries that span more
+// than kExpandSpan rows (a long run of empty ones) are searched for one by one:
+// 16 searches per thread against one step per 256 rows.
+constexpr uint32_t kExpandSpan = 1u << 16;
+// Largest u in [lo, hi] with row[u] <= e: the row that holds entry e.
+__device__ __forceinline__ uint32_t row_of_entry(const uint32_t *row, uint32_t lo, uint32_t hi, uint32_t e) {
+    while (lo < hi) {
+        const uint32_t mid = lo + (hi - lo + 1) / 2;
+        if (__ldg(row + mid) <= e) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
 __global__ void __launch_bounds__(kRadixThreads) expand_rows_kernel(const uint32_t *row, uint32_t nv, uint64_t ne,
                                                                     uint32_t *src) {
     __shared__ uint32_t mark[kRadixTile];
@@ -763,19 +775,17 @@ __global__ void __launch_bounds__(kRadixThreads) expand_rows_kernel(const uint32
     const uint64_t tiles = (ne + kRadixTile - 1) / kRadixTile;
     for (uint64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
         const uint64_t e0 = t * kRadixTile, e1 = min(ne, e0 + kRadixTile);
-        if (threadIdx.x < 2) {  // largest u with row[u] <= e: the row of the tile's first and last entry
-            const uint32_t e = (uint32_t)(threadIdx.x == 0 ? e0 : e1 - 1);
-            uint32_t lo = 0, hi = nv - 1;
-            while (lo < hi) {
-                const uint32_t mid = lo + (hi - lo + 1) / 2;
-                if (__ldg(row + mid) <= e) lo = mid;
-                else hi = mid - 1;
-            }
-            span[threadIdx.x] = lo;
-        }
+        if (threadIdx.x < 2)  // rows of the tile's first and last entry
+            span[threadIdx.x] = row_of_entry(row, 0, nv - 1, (uint32_t)(threadIdx.x == 0 ? e0 : e1 - 1));
         for (uint32_t i = threadIdx.x; i < kRadixTile; i += kRadixThreads) mark[i] = 0;
         __syncthreads();
         const uint32_t r0 = span[0], r1 = span[1];
+        if (r1 - r0 > kExpandSpan) {
+            for (uint64_t e = e0 + threadIdx.x; e < e1; e += kRadixThreads)
+                src[e] = row_of_entry(row, r0, r1, (uint32_t)e);
+            __syncthreads();
+            continue;
+        }
         for (uint64_t r = (uint64_t)r0 + threadIdx.x; r <= r1; r += kRadixThreads) {
             const uint32_t b = __ldg(row + r);
             if (b < __ldg(row + r + 1)) mark[b > e0 ? (uint32_t)(b - e0) : 0u] = (uint32_t)(r - r0);

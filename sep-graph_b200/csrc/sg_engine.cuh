@@ -193,8 +193,8 @@ struct KArgs {
     uint32_t *sort_counts = nullptr;
     // Edge-tiled pull (functors with PullReduce, unweighted, topology-driven;
     // min-relax functors): tile_row[t] = the in-edge row holding CSC edge
-    // t * kPullTileEdges (ceil(E / kPullTileEdges) + 1 entries, the last =
-    // V - 1), filled at the launch's start or in its first pull round; null =
+    // t * kPullTileEdges (ceil(E / kPullTileEdges) + 1 entries, the last = the
+    // row of the last edge), filled at the launch's start or in its first pull round; null =
     // the destination-per-lane pull is used instead.
     uint32_t *tile_row = nullptr;
     // Pull over destinations: (vertex, first in-edge, in-edges, -) chunks of
@@ -220,6 +220,12 @@ constexpr uint32_t kPullTileEdges = 256;
 // Row segments of a tile that are combined in shared memory first; a tile with
 // more goes row by row.
 constexpr uint32_t kPullTileRows = 96;
+// Rows a tile may span and still have them ranked 32 at a time (32 dependent
+// steps); lanes of a tile with a longer run of empty rows search for theirs
+// (10 steps and more per row of a lane).  Without the limit one warp stepped
+// through all of them: 20 PageRank pull rounds on R-MAT of 2^20 vertices with
+// 2^22 unused ids between its halves 1289 ms, with it 3.7 (2.5 without the ids).
+constexpr uint32_t kPullTileSpan = 1024;
 
 // Leader-only policy state (RunningInfo), lives in block 0 / thread 0.
 struct PolicyState {
@@ -2363,16 +2369,21 @@ struct EngineKernel {
         const uint32_t V = a.csc.nnodes, E = a.csc.nedges;
         const uint32_t T = (E + kPullTileEdges - 1) / kPullTileEdges;
         for (uint32_t t = gthread(); t <= T; t += nthreads())
-            a.tile_row[t] = (t == T || V == 0) ? (V ? V - 1 : 0) : row_of(a.csc.col_start, 0, V - 1, t * kPullTileEdges);
+            a.tile_row[t] = T == 0 ? 0u : row_of(a.csc.col_start, 0, V - 1, t < T ? t * kPullTileEdges : E - 1);
     }
 
     // The rows of a tile of edges [t0, t0 + t1): segment 0 is row rlo's share,
     // segment k the k-th row that starts inside the tile (segrow = its distance
     // from rlo; its first edge is marked).  Returns the segments; from
-    // kPullTileRows on they are not all recorded.  All 32 lanes call.
+    // kPullTileRows on (also returned for a tile that spans more than
+    // kPullTileSpan rows) they are not all recorded.  All 32 lanes call.
     static __device__ __forceinline__ uint32_t rank_tile_rows(WarpLB<TB> &w, const uint32_t *crow, uint32_t rlo,
                                                               uint32_t rhi, uint32_t t0, uint32_t t1) {
         const uint32_t lane = dev::lane_id();
+        if (rhi - rlo > kPullTileSpan) {
+            __syncwarp();  // the tile's values are read: the next tile may overwrite them
+            return kPullTileRows;
+        }
         if (lane < 8) w.mark[lane] = 0;
         if (lane == 0) w.segrow[0] = 0;
         __syncwarp();

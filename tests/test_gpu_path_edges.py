@@ -161,6 +161,51 @@ def test_pagerank_tiles_and_dense_push(ctx, nv, m, variant, no_csc):
     G.close()
 
 
+def _gap(nv, m, at, gap, seed):
+    """A random graph whose ids from `at` on are moved up by `gap` unused ones."""
+    s, d = _random(nv, m, seed)
+    up = lambda x: np.where(x >= at, x + gap, x).astype(np.uint32)
+    return nv + gap, up(s), up(d)
+
+
+# gaps around the rows a tile ranks (1024) and the rows an entry tile walks (65536), at the start, inside and at the end
+@pytest.mark.parametrize("gap", [1000, 1030, 65500, 70000])
+@pytest.mark.parametrize("at", [0, 1500, 3000])
+def test_runs_of_unused_ids(ctx, gap, at):
+    nv, s, d = _gap(3000, 40000, at, gap, gap + at)
+    w = np.random.default_rng(gap).integers(1, 1000, len(s)).astype(np.uint32)
+    src = int(s[0])
+    off, idx, ww = _csr(nv, s, d, w)
+    G = ctx.graph_from_csr(off, idx, ww)
+    for variant in ("async_pull_dd", "sync_pull_td", "auto"):
+        assert np.array_equal(G.sssp(src, variant=variant, max_iteration=100000)[0], oracle.sssp(off, idx, ww, src))
+    bc, sigma, _ = G.bc(src, variant="async_pull_dd")
+    want, sig, _ = oracle.bc_f64(off, idx, src)
+    assert np.array_equal(sigma.astype(np.float64), sig)
+    assert np.all(np.abs(bc - want) <= 1e-4 * np.abs(want) + 1e-5)
+    want = oracle.pagerank_fixed_point_f64(off, idx)[0]
+    for variant in ("sync_pull_td", "async_push_dd"):
+        r = G.pagerank(variant=variant, pr_error=1e-8, max_iteration=100000, lb_push="fine")[0].astype(np.float64)
+        assert np.abs(r / r.sum() - want / want.sum()).sum() <= 1e-6
+    coff, cidx, cw = G.copy_out(csc=True)
+    G.close()
+    tc = oracle.csr_tocsc(off, idx, ww)
+    assert np.array_equal(coff, tc[0]) and np.array_equal(cidx, tc[1]) and np.array_equal(cw, tc[2])
+
+
+def test_unused_ids_cost_their_passes_only(ctx):
+    """10 pull rounds with 4 M unused ids between two halves of a graph: a few passes over the ids (about 0.2 ms a
+    round), where a warp that steps through them 32 at a time takes over 60 ms a round."""
+    ms = []
+    for gap in (0, 1 << 22):
+        nv, s, d = _gap(65536, 1 << 20, 32768, gap, 5)
+        off, idx, _ = _csr(nv, s, d)
+        G = ctx.graph_from_csr(off, idx)
+        ms.append(min(G.pagerank(variant="sync_pull_td", max_iteration=10)[1].time_kernel_ms for _ in range(3)))
+        G.close()
+    assert ms[1] < ms[0] + 50, ms
+
+
 # entries around one radix tile (4096), ids around a digit (8 bits) and several
 BUILDS = [(1, 5), (2, 4095), (255, 4096), (256, 4097), (257, 8192), (65536, 8193), (65537, 20000), (70000, 3)]
 
