@@ -43,8 +43,8 @@ struct BCBackArgs {
     unsigned long long timeout_ns;
 };
 
-__device__ __forceinline__ float bc_q(const BCBackArgs &a, uint32_t v, float delta) {
-    return (float)((1.0 + (double)delta) / (double)__ldcg(a.sigma + v));
+__device__ __forceinline__ float bc_q(unsigned long long sigma, float delta) {
+    return (float)((1.0 + (double)delta) / (double)sigma);
 }
 
 // Sum of q over the out-edges [k, end) taken `step` apart that lead to `depth`,
@@ -65,11 +65,12 @@ __device__ __forceinline__ float bc_sum(const BCBackArgs &a, uint32_t k, uint32_
     return s;
 }
 
-// Dependency of v from its sum, and its record for the level above.
-__device__ __forceinline__ void bc_finish(const BCBackArgs &a, uint32_t v, float sum, uint32_t depth) {
-    const float d = (float)((double)__ldcg(a.sigma + v) * (double)sum);
+// Dependency of v (sigma paths) from its sum, and its record for the level above.
+__device__ __forceinline__ void bc_finish(const BCBackArgs &a, uint32_t v, unsigned long long sigma, float sum,
+                                          uint32_t depth) {
+    const float d = (float)((double)sigma * (double)sum);
     a.delta[v] = d;
-    a.rec[v] = make_uint2(depth, __float_as_uint(bc_q(a, v, d)));
+    a.rec[v] = make_uint2(depth, __float_as_uint(bc_q(sigma, d)));
 }
 
 // The whole backward pass for one query, run by `nt` threads numbered from
@@ -80,10 +81,12 @@ __device__ bool backward(const BCBackArgs &a, uint32_t gt, uint32_t nt, Sync &&s
     const uint32_t lane = dev::lane_id();
     const uint32_t gw = gt >> 5, nw = nt >> 5;
     uint32_t chunk0 = 0;  // first chunk of the level at hand
-    // chunks of the split vertices of depth d, after `base` earlier ones
+    // chunks of the split vertices of depth d, after `base` earlier ones; from
+    // the last thread down, so that on a level smaller than the team other warps
+    // sum meanwhile
     auto list_chunks = [&](uint32_t d, uint32_t base) {
         const uint32_t b = __ldcg(a.ends + d - 1), e = __ldcg(a.ends + d);
-        for (uint32_t i = b + gt; i < e; i += nt) {
+        for (uint32_t i = b + (nt - 1 - gt); i < e; i += nt) {
             const uint32_t v = __ldcg(a.stack + i);
             const uint32_t beg = __ldg(a.row + v), deg = __ldg(a.row + v + 1) - beg;
             if (deg <= kBcBigDegree) continue;
@@ -101,7 +104,7 @@ __device__ bool backward(const BCBackArgs &a, uint32_t gt, uint32_t nt, Sync &&s
         // vertices below max_depth have no successors: delta 0, q = 1 / sigma
         for (uint32_t v = gt; v < a.nv; v += nt) {
             const uint32_t lv = __ldcg(a.level + v);
-            a.rec[v] = make_uint2(lv, lv != 0xffffffffu && lv > a.max_depth ? __float_as_uint(bc_q(a, v, 0.f)) : 0u);
+            a.rec[v] = make_uint2(lv, lv != 0xffffffffu && lv > a.max_depth ? __float_as_uint(bc_q(__ldcg(a.sigma + v), 0.f)) : 0u);
         }
         list_chunks(a.max_depth, 0);
         if (!sync()) return false;
@@ -118,13 +121,15 @@ __device__ bool backward(const BCBackArgs &a, uint32_t gt, uint32_t nt, Sync &&s
             const uint32_t i = base + lane;
             const bool valid = i < e;
             uint32_t v = 0, beg = 0, deg = 0;
+            unsigned long long sigma = 0;  // in flight with the row: a trip less at the end of the chain
             if (valid) {
                 v = __ldcg(a.stack + i);
                 beg = __ldg(a.row + v);
                 deg = __ldg(a.row + v + 1) - beg;
+                sigma = __ldcg(a.sigma + v);
             }
             const bool mid = valid && deg <= kBcBigDegree && deg > 32;
-            if (valid && deg <= 32) bc_finish(a, v, bc_sum(a, beg, beg + deg, 1, d + 1), d);
+            if (valid && deg <= 32) bc_finish(a, v, sigma, bc_sum(a, beg, beg + deg, 1, d + 1), d);
             uint32_t m = __ballot_sync(dev::kFullMask, mid);
             while (m) {
                 const uint32_t j = __ffs(m) - 1;
@@ -132,8 +137,9 @@ __device__ bool backward(const BCBackArgs &a, uint32_t gt, uint32_t nt, Sync &&s
                 const uint32_t vj = __shfl_sync(dev::kFullMask, v, j);
                 const uint32_t bj = __shfl_sync(dev::kFullMask, beg, j);
                 const uint32_t dj = __shfl_sync(dev::kFullMask, deg, j);
+                const unsigned long long sj = __shfl_sync(dev::kFullMask, sigma, j);
                 const float s = dev::warp_sum(bc_sum(a, bj + lane, bj + dj, 32, d + 1));
-                if (lane == 0) bc_finish(a, vj, s, d);
+                if (lane == 0) bc_finish(a, vj, sj, s, d);
             }
         }
         if (d > 1) list_chunks(d - 1, end);
@@ -141,7 +147,7 @@ __device__ bool backward(const BCBackArgs &a, uint32_t gt, uint32_t nt, Sync &&s
         if (end > chunk0) {  // the same in every thread
             for (uint32_t c = chunk0 + gt; c < end; c += nt) {
                 const uint4 ch = __ldcg(a.chunks + c);
-                if (ch.w) bc_finish(a, ch.x, __ldcg(a.delta + ch.x), d);
+                if (ch.w) bc_finish(a, ch.x, __ldcg(a.sigma + ch.x), __ldcg(a.delta + ch.x), d);
             }
             if (!sync()) return false;
             chunk0 = end;
