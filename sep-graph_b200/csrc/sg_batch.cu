@@ -775,7 +775,8 @@ using BCApp = apps::BCForward<uint32_t, uint32_t, graphs::NoWeight>;
 // same round loop as a single query) and then the backward pass over its own
 // level stack with team barriers, and writes delta * 0.5 to the query's
 // output.  Forward and backward of different queries overlap across teams.
-__global__ void __launch_bounds__(engine::kBlockThreads, 4)
+template <bool kFew>
+__global__ void __launch_bounds__(engine::kBlockThreads, kFew ? 3 : 4)
     batched_bc_kernel(const engine::BatchQuery<BCApp, uint32_t> *queries, uint32_t nq,
                       const engine::TeamSpace<uint32_t> *spaces, const BCTeam *bcs, float *const *outs,
                       uint32_t team_blocks, uint32_t *next_query, engine::BatchResult *results, engine::Params p) {
@@ -946,14 +947,30 @@ sg_status prepare_batch(sg_ctx *ctx, sgb::Workspace &ws, std::vector<engine::Bat
     constexpr bool kBC = std::is_same<App, BCApp>::value;
     B.bc = kBC;
     B.value_bytes = sizeof(TV);
-    B.kernel = kBC ? (const void *)batched_bc_kernel : (const void *)batched_engine_kernel<App, TV, TB, TW>;
-    static std::atomic<int> occupancy[2] = {{0}, {0}};  // per template instantiation: all variants, push
+    // unweighted batches take three blocks per SM when every graph is sparse (see
+    // few_blocks), four otherwise: 32 BFS on the 512^2 grid 25.1 ms with three,
+    // 26.1 with four; on symmetric RMAT-18, pushing, 2.72 and 2.28
+    bool sparse = true;
+    for (auto *g : graphs) sparse = sparse && (double)g->ne < kFewBlocksDegree * g->nv;
+    // per template instantiation: all variants, push, all variants for few blocks
+    static std::atomic<int> occupancy[3] = {{0}, {0}, {0}};
     int which = 0;
-    if constexpr (specialised<App, TB, TW>(V_ASYNC_PUSH_DD))
-        if (p.forced == V_ASYNC_PUSH_DD) {
-            B.kernel = (const void *)batched_engine_kernel<App, TV, TB, TW, V_ASYNC_PUSH_DD>;
-            which = 1;
-        }
+    if constexpr (kBC) {
+        which = sparse ? 2 : 0;
+        B.kernel = sparse ? (const void *)batched_bc_kernel<true> : (const void *)batched_bc_kernel<false>;
+    } else {
+        B.kernel = (const void *)batched_engine_kernel<App, TV, TB, TW>;
+        if constexpr (has_few_blocks_kernel<App, TB, TW>())
+            if (sparse) {
+                B.kernel = (const void *)batched_engine_kernel<App, TV, TB, TW, -1, true>;
+                which = 2;
+            }
+        if constexpr (specialised<App, TB, TW>(V_ASYNC_PUSH_DD))
+            if (p.forced == V_ASYNC_PUSH_DD) {
+                B.kernel = (const void *)batched_engine_kernel<App, TV, TB, TW, V_ASYNC_PUSH_DD>;
+                which = 1;
+            }
+    }
     int max_bps = 0;
     SG_TRY_CUDA(ctx, sgb::occupancy_once(occupancy[which], B.kernel, kBlockThreads, &max_bps));
     const int bps =

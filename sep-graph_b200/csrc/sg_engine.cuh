@@ -3172,19 +3172,38 @@ constexpr bool specialised(int v) {
     return (v == V_ASYNC_PUSH_DD && (reduce || has_min_relax<App, TB, TW>::value)) || (v == V_SYNC_PULL_TD && reduce);
 }
 
-// Resident blocks per SM that the kernels are compiled for (registers): the
-// unweighted functors' rounds fit 51 registers, push PageRank with the tiles of
-// its dense rounds takes 64 (1,000,003 vertices 15.9 -> 14.6 ms), relaxation with
-// eight edges in flight per lane 80 (at 64, four blocks, it spills: 256 SSSP in
-// one call 50.5 -> 55.8 ms).
-template <typename TW, int kForced>
+// Resident blocks per SM that the kernels are compiled for (registers): push
+// PageRank with the tiles of its dense rounds takes 64 registers (1,000,003
+// vertices 15.9 -> 14.6 ms), relaxation with eight edges in flight per lane 80
+// (at 64, four blocks, it spills: 256 SSSP in one call 50.5 -> 55.8 ms).  The
+// unweighted functors' kernel of all variants needs 80 and is compiled twice
+// (see few_blocks): with five blocks of 48, spilling, and with three (kFew).
+template <typename TW, int kForced, bool kFew = false>
 constexpr int min_blocks() {
-    return !std::is_same<TW, graphs::NoWeight>::value ? 3 : kForced == V_ASYNC_PUSH_DD ? 4 : 5;
+    return kFew || !std::is_same<TW, graphs::NoWeight>::value ? 3 : kForced == V_ASYNC_PUSH_DD ? 4 : 5;
+}
+
+// Which of the two: a round of a small or sparse graph is one chain of memory
+// trips and a spilled register read back after the barrier is a trip more, a
+// dense round of a large graph wants the blocks, a push round sooner than a pull
+// round.  BFS, ms with five and with three blocks: grids of 512^2 and 1500^2
+// vertices 7.9 / 6.5 and 31.6 / 24.9; symmetric RMAT-18 (7 M edges), 20 (29 M), 21
+// (60 M) and 22 (123 M) by the hybrid policy 0.171 / 0.158, 0.245 / 0.235, 0.348 /
+// 0.352 and 0.83 / 0.99, pushing 0.263 / 0.258, 0.481 / 0.514 and 0.737 / 0.841.
+constexpr uint64_t kFewBlocksEdges = 1ull << 25, kFewBlocksPushEdges = 1ull << 24;
+constexpr double kFewBlocksDegree = 8.0;
+inline bool few_blocks(uint32_t nv, uint64_t ne, bool push) {
+    return ne < (push ? kFewBlocksPushEdges : kFewBlocksEdges) || (double)ne < kFewBlocksDegree * nv;
+}
+// The unweighted traversals; PageRank's rounds go over all edges at any size.
+template <typename App, typename TB, typename TW>
+constexpr bool has_few_blocks_kernel() {
+    return std::is_same<TW, graphs::NoWeight>::value && !has_pull_reduce<App, TB>::value;
 }
 
 // One query: the whole cooperative grid is the team.
-template <typename App, typename TV, typename TB, typename TW, int kForced = -1>
-__global__ void __launch_bounds__(kBlockThreads, min_blocks<TW, kForced>())
+template <typename App, typename TV, typename TB, typename TW, int kForced = -1, bool kFew = false>
+__global__ void __launch_bounds__(kBlockThreads, min_blocks<TW, kForced, kFew>())
     hybrid_engine_kernel(const App app_in, KArgs<TV, TB, TW> a) {
     set_team(blockIdx.x, gridDim.x, a.ctrl);
     run_instance<App, TV, TB, TW, kForced>(app_in, a);
@@ -3244,8 +3263,8 @@ __device__ __forceinline__ void write_result(BatchResult *r, const Ctrl *c, uint
 // team-local barrier, records its result and moves on.  Per-query frontiers
 // and state never leave the device; the batch is one launch (capturable in a
 // CUDA graph).
-template <typename App, typename TV, typename TB, typename TW, int kForced = -1>
-__global__ void __launch_bounds__(kBlockThreads, min_blocks<TW, kForced>() < 4 ? min_blocks<TW, kForced>() : 4)
+template <typename App, typename TV, typename TB, typename TW, int kForced = -1, bool kFew = false>
+__global__ void __launch_bounds__(kBlockThreads, min_blocks<TW, kForced, kFew>() < 4 ? min_blocks<TW, kForced, kFew>() : 4)
     batched_engine_kernel(const BatchQuery<App, TV> *queries, uint32_t nq, const TeamSpace<TB> *spaces,
                           uint32_t team_blocks, uint32_t *next_query, BatchResult *results, Params p) {
     const uint32_t team = blockIdx.x / team_blocks;

@@ -197,7 +197,8 @@ extern "C" sg_status sg_bfs_noalloc(const uint32_t *offsets, const uint32_t *ind
     // State that must start at zero: the control block and the heavy-vertex
     // tables (bitmaps are cleared by the kernel's first phase).
     cudaError_t e = cudaMemsetAsync(base + kOffHeavy, 0, kOffCtrl + sizeof(Ctrl) - kOffHeavy, s);
-    auto kernel = engine::hybrid_engine_kernel<BfsApp, uint32_t, uint32_t, graphs::NoWeight>;
+    static_assert(kNoAllocMaxEdges < engine::kFewBlocksPushEdges, "the kernel for small graphs");
+    auto kernel = engine::hybrid_engine_kernel<BfsApp, uint32_t, uint32_t, graphs::NoWeight, -1, true>;
     int bps = 0, sms = 0;
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel, engine::kBlockThreads, 0);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -527,8 +527,14 @@ sg_status run_engine(sg_graph *g, App app, const EngineConfig &cfg, TV *value, T
     app.m_p_current_round = &a.ctrl->rs.round;
 
     const void *kernel = (const void *)hybrid_engine_kernel<App, TV, TB, TW>;
-    static std::atomic<int> occupancy[3] = {{0}, {0}, {0}};  // per template instantiation: all variants, push, pull
+    // per template instantiation: all variants, push, pull, all variants for few blocks
+    static std::atomic<int> occupancy[4] = {{0}, {0}, {0}, {0}};
     int which = 0;
+    if constexpr (has_few_blocks_kernel<App, TB, TW>())
+        if (few_blocks(nv, ne, cfg.forced >= 0 && !is_pull(cfg.forced))) {
+            kernel = (const void *)hybrid_engine_kernel<App, TV, TB, TW, -1, true>;
+            which = 3;
+        }
     if constexpr (specialised<App, TB, TW>(V_ASYNC_PUSH_DD))
         if (cfg.forced == V_ASYNC_PUSH_DD && !cfg.trace) {
             kernel = (const void *)hybrid_engine_kernel<App, TV, TB, TW, V_ASYNC_PUSH_DD>;

@@ -161,6 +161,39 @@ def test_pagerank_tiles_and_dense_push(ctx, nv, m, variant, no_csc):
     G.close()
 
 
+@pytest.mark.parametrize("variant", ["auto", "async_push_dd", "async_pull_dd"])
+def test_batches_by_density(ctx, variant):
+    """Batches of sparse graphs alone, of dense ones alone and of both take different kernels."""
+    graphs = []
+    for nv, s, d in (_cliques(40, 12), _cliques(3000, 3)):
+        off, idx, _ = _csr(nv, s, d)
+        graphs.append((ctx.graph_from_csr(off, idx, symmetric=True), off, idx))
+    kw = dict(variant=variant, max_iteration=100000)
+    for picks in ([0], [1], [0, 1]):
+        queries = [(graphs[g][0], src) for g in picks for src in (0, 7, 450)]
+        levels = ctx.bfs_batch(queries, **kw)[0]
+        deps = ctx.bc_batch(queries, **kw)[0]
+        for (g, src), lv, dep in zip([(g, src) for g in picks for src in (0, 7, 450)], levels, deps):
+            _, off, idx = graphs[g]
+            assert np.array_equal(lv, oracle.bfs(off, idx, src))
+            want = oracle.bc_f64(off, idx, src)[0]
+            assert np.all(np.abs(dep - want) <= 1e-4 * np.abs(want) + 1e-5)
+    for G, _, _ in graphs:
+        G.close()
+
+
+@pytest.mark.parametrize("variant", ["auto", "async_push_dd"])
+def test_bc_above_the_dense_size(ctx, variant):
+    h = sg.HostGraph.rmat(21, 16, symmetric=True, seed=1)
+    G = ctx.graph(h, symmetric=True)
+    src = int(h.pick_sources(1, 3)[0])
+    bc, sigma, _ = G.bc(src, variant=variant)
+    want, sig, _ = oracle.bc_f64(h.offsets, h.indices, src)
+    assert np.array_equal(sigma.astype(np.float64), sig)
+    assert np.all(np.abs(bc - want) <= 1e-4 * np.abs(want) + 1e-5)
+    G.close()
+
+
 def _gap(nv, m, at, gap, seed):
     """A random graph whose ids from `at` on are moved up by `gap` unused ones."""
     s, d = _random(nv, m, seed)
