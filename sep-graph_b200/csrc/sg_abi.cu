@@ -203,7 +203,7 @@ sg_status sg_destroy(sg_ctx *ctx) {
     cudaStreamSynchronize(ctx->stream);
     sgb::persist_release(ctx);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
-    if (ctx->spare_arena) cudaFree(ctx->spare_arena);
+    sgb::release_spare(ctx);
     delete ctx->batch_ws;  // frees on the context's stream and waits for it
     delete ctx->graph_ws;
     if (cudaMemPool_t pool = sgb::device_pool(ctx->device)) cudaMemPoolTrimTo(pool, 0);
@@ -288,7 +288,7 @@ sg_status create_graph(sg_ctx *ctx, uint32_t nv, uint64_t ne, const uint32_t *of
         ctx->spare_arena = nullptr;
         ctx->spare_bytes = 0;
     } else {
-        e = cudaMalloc(&g->arena, total);
+        e = arena_alloc(ctx, &g->arena, total);
         if (e != cudaSuccess) {
             delete g;
             return sgb::cuda_status(ctx, e, "graph arena");
@@ -319,7 +319,7 @@ sg_status create_graph(sg_ctx *ctx, uint32_t nv, uint64_t ne, const uint32_t *of
     uint32_t bad_dst = 0;
     auto fail = [&](sg_status st) {
         cudaStreamSynchronize(s);
-        cudaFree(g->arena);
+        arena_free(ctx, g->arena, g->arena_bytes);
         delete g;
         return st;
     };
@@ -380,11 +380,11 @@ sg_status sg_graph_destroy(sg_graph *g) {
     if (g->arena) {
         // keep the larger of this arena and the context's spare for the next graph
         if (!ctx->spare_arena || ctx->spare_bytes < g->arena_bytes) {
-            if (ctx->spare_arena) cudaFree(ctx->spare_arena);
+            sgb::release_spare(ctx);
             ctx->spare_arena = g->arena;
             ctx->spare_bytes = g->arena_bytes;
         } else {
-            cudaFree(g->arena);
+            sgb::arena_free(ctx, g->arena, g->arena_bytes);
         }
     }
     ctx->live_graphs--;
@@ -396,9 +396,7 @@ sg_status sg_ctx_release_cached(sg_ctx *ctx) {
     if (!ctx) return SG_ERR_INVALID_ARG;
     DeviceGuard dg(ctx->device);
     SG_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (ctx->spare_arena) cudaFree(ctx->spare_arena);
-    ctx->spare_arena = nullptr;
-    ctx->spare_bytes = 0;
+    sgb::release_spare(ctx);
     delete ctx->graph_ws;
     ctx->graph_ws = nullptr;
     delete ctx->batch_ws;
@@ -407,6 +405,15 @@ sg_status sg_ctx_release_cached(sg_ctx *ctx) {
 }
 
 }  // extern "C"
+
+extern "C" sg_status sg_debug_build_memory(sg_ctx *ctx, int counting, uint64_t limit, uint64_t *peak) {
+    if (!ctx) return SG_ERR_INVALID_ARG;
+    ctx->build_by_counting = counting != 0;
+    ctx->mem.limit = limit ? (size_t)limit : ~size_t(0);
+    if (peak) *peak = ctx->mem.peak;
+    ctx->mem.peak = ctx->mem.used;
+    return SG_OK;
+}
 
 sg_ctx *sgb::graph_context(const sg_graph *g) { return g ? g->ctx : nullptr; }
 double sgb::graph_weight_sum(const sg_graph *g) { return g ? g->weight_sum : 0.0; }

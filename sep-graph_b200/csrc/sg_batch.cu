@@ -634,7 +634,7 @@ sg_status sgb::msbfs_on(sg_ctx *ctx, sg_graph *g, const uint32_t *sources, uint3
     if (row_outs)
         for (uint32_t i = 0; i < nsrc; ++i)
             if (!row_outs[i]) return SG_ERR_INVALID_ARG;
-    if (!ctx->batch_ws) ctx->batch_ws = new sgb::Workspace(&ctx->stream, sgb::device_pool(ctx->device));
+    if (!ctx->batch_ws) ctx->batch_ws = new sgb::Workspace(ctx);
     for (uint32_t i = 0; i < nsrc; ++i)
         if (sources[i] >= g->nv) return sgb::set_error(ctx, SG_ERR_INVALID_ARG, "source %u out of range", sources[i]);
     int prev = -1;
@@ -1227,7 +1227,7 @@ template <typename App, typename TV, typename TB, typename TW>
 sg_status run_batch(sg_ctx *ctx, std::vector<engine::BatchQuery<App, TV>> qs, const std::vector<sg_graph *> &graphs,
                     const std::vector<void *> &outs, const sg_options &o, engine::Params p, sg_stats *stats,
                     float *per_query_ms) {
-    if (!ctx->batch_ws) ctx->batch_ws = new sgb::Workspace(&ctx->stream, sgb::device_pool(ctx->device));
+    if (!ctx->batch_ws) ctx->batch_ws = new sgb::Workspace(ctx);
     BatchBuild B;
     sg_status st = prepare_batch<App, TV, TB, TW>(ctx, *ctx->batch_ws, std::move(qs), graphs, outs, o, p, false, B);
     if (st != SG_OK) return st;

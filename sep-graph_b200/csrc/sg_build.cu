@@ -18,7 +18,7 @@
 //    entry (it holds the entry's input position), so the result never depends
 //    on the scatter order.  It needs 4 or 8 bytes of scratch per entry where
 //    the radix sort needs 16 (24 with a payload), and runs when the device
-//    cannot give that.
+//    cannot give that or what comes after it (build_rows, arena_alloc).
 // Measured on B200, RMAT-21 raw weighted edges (33.5 M, self-loops and
 // duplicates dropped, rows ordered) to a CSR with its in-edge view: 9.25 ms by counting, 4.25 ms by the radix sort.
 //
@@ -56,10 +56,7 @@ __device__ __forceinline__ K key_max() {
     return (K)~(K)0;
 }
 
-inline Workspace &build_ws(sg_ctx *ctx) {
-    if (!ctx->graph_ws) ctx->graph_ws = new Workspace(&ctx->stream, device_pool(ctx->device));
-    return *ctx->graph_ws;
-}
+inline Workspace &build_ws(sg_ctx *ctx) { return graph_ws(ctx); }
 
 // Temporary device buffers of one call, named in the context's grow-only
 // scratch (released by sg_ctx_release_cached): repeated builds and
@@ -68,16 +65,24 @@ inline Workspace &build_ws(sg_ctx *ctx) {
 // so buffers whose lifetimes overlap never share a name; a later call with
 // the same prefix reuses the buffers of an earlier one, which is finished by
 // then (all work of a context is ordered on its stream).
-struct Tmp {
+struct Tmp : BuildBuffers {
     sg_ctx *ctx;
-    const char *prefix;
-    unsigned n = 0;
-    Tmp(sg_ctx *c, const char *p) : ctx(c), prefix(p) {}
+    bool sorting = false;  // a radix sort of this call is using its scratch
+    Tmp(sg_ctx *c, const char *p) : BuildBuffers{p}, ctx(c) { ctx->building.push_back(this); }
+    ~Tmp() { ctx->building.pop_back(); }
+    Tmp(const Tmp &) = delete;
+    Tmp &operator=(const Tmp &) = delete;
+    // Without room, once more without the scratch of a sort that has ended.
     template <class T>
     cudaError_t alloc(T **p, uint64_t count) {
-        char name[48];
-        std::snprintf(name, sizeof name, "gb_%s_%u", prefix, n++);
-        return build_ws(ctx).get(name, (size_t)std::max<uint64_t>(count, 1), p);
+        const std::string id = name(n++);
+        const size_t c = (size_t)std::max<uint64_t>(count, 1);
+        cudaError_t e = build_ws(ctx).get(id.c_str(), c, p);
+        if (e == cudaErrorMemoryAllocation && !sorting) {
+            release_build_scratch(ctx);
+            e = build_ws(ctx).get(id.c_str(), c, p);
+        }
+        return e;
     }
 };
 
@@ -916,13 +921,11 @@ struct BuiltCsr {
 // `dedup`, else by row alone; `dedup` keeps the first entry of every (row,
 // column).  Entries of `trusted` lists are all kept and in range.  The CSR goes
 // to dest (nv + 1 offsets, columns and weights) or to temporaries of the call.
-// SG_ERR_OUT_OF_MEMORY when the device cannot give the scratch (nothing has
-// run then).
 struct CsrDest {
     uint32_t *row, *col, *w;
 };
-sg_status build_rows_radix(sg_ctx *ctx, Tmp &tmp, const EdgeList &el, bool sorted, bool dedup, bool trusted,
-                           const CsrDest *dest, BuiltCsr *out) {
+sg_status sort_rows_radix(sg_ctx *ctx, Tmp &tmp, const EdgeList &el, bool sorted, bool dedup, bool trusted,
+                          const CsrDest *dest, BuiltCsr *out) {
     const cudaStream_t s = ctx->stream;
     const uint32_t nv = el.nv;
     const uint64_t n_in = el.m << el.rs;
@@ -949,11 +952,7 @@ sg_status build_rows_radix(sg_ctx *ctx, Tmp &tmp, const EdgeList &el, bool sorte
         if (twice && (e = get("gb_rx_alive", nwords, &alive)) != cudaSuccess) return e;
         return get("gb_rx_bad", 1, &bad);
     };
-    if (const cudaError_t e = scratch()) {
-        cudaGetLastError();
-        ws.drop("gb_rx_");  // the counting path may need the room
-        return cuda_status(ctx, e, "radix sort scratch");
-    }
+    if (const cudaError_t e = scratch()) return cuda_status(ctx, e, "radix sort scratch");
     constexpr size_t smem = sizeof(RadixShared);
     SG_TRY_CUDA(ctx, cudaMemsetAsync(bad, 0xff, sizeof *bad, s));
 
@@ -1058,6 +1057,22 @@ sg_status build_rows_radix(sg_ctx *ctx, Tmp &tmp, const EdgeList &el, bool sorte
     out->w = w;
     out->ne = ne;
     return SG_OK;
+}
+
+// The same, SG_ERR_OUT_OF_MEMORY without scratch and temporaries when the device
+// has no room for them: counting may do with what that leaves.
+sg_status build_rows_radix(sg_ctx *ctx, Tmp &tmp, const EdgeList &el, bool sorted, bool dedup, bool trusted,
+                           const CsrDest *dest, BuiltCsr *out) {
+    if (ctx->build_by_counting) return SG_ERR_OUT_OF_MEMORY;
+    const unsigned first = tmp.n;
+    tmp.sorting = true;
+    const sg_status st = sort_rows_radix(ctx, tmp, el, sorted, dedup, trusted, dest, out);
+    tmp.sorting = false;
+    if (st == SG_ERR_OUT_OF_MEMORY) {
+        tmp.n = first;
+        release_build_scratch(ctx);
+    }
+    return st;
 }
 
 // Edge list -> CSR by counting: count, scan, scatter, sort rows by
@@ -1169,17 +1184,16 @@ sg_status device_transpose(sg_ctx *ctx, uint32_t nv, uint64_t ne, const uint32_t
     // the edges as (destination, source) entries in CSR order, ordered by destination
     uint32_t *src = nullptr;
     sg_status rst = SG_ERR_OUT_OF_MEMORY;
-    if (build_ws(ctx).get("gb_rx_src", (size_t)std::max<uint64_t>(ne, 1), &src) == cudaSuccess) {
+    if (!ctx->build_by_counting &&
+        build_ws(ctx).get("gb_rx_src", (size_t)std::max<uint64_t>(ne, 1), &src) == cudaSuccess) {
         if ((rst = enqueue_expand_rows(ctx, row, nv, ne, src)) != SG_OK) return rst;
         const EdgeList el{col, src, w, ne, nv, 0u, false};
         const CsrDest dest{crow, ccol, cw};
         BuiltCsr built;
         rst = build_rows_radix(ctx, tmp, el, false, false, true, &dest, &built);
-    } else {
-        cudaGetLastError();
     }
     if (rst != SG_ERR_OUT_OF_MEMORY) return rst;
-    build_ws(ctx).drop("gb_rx_");
+    release_build_scratch(ctx);
     uint32_t *cnt;
     SG_TRY_CUDA(ctx, tmp.alloc(&cnt, (uint64_t)nv + 1));
     SG_TRY_CUDA(ctx, cudaMemsetAsync(cnt, 0, 4ull * (nv + 1), s));
@@ -1241,7 +1255,7 @@ sg_status symmetric_weighted_csc(sg_ctx *ctx, sg_graph *g) {
     const size_t b_row = al(4ull * (nv + 1)), b_col = al(4ull * std::max<uint64_t>(ne, 1));
     const size_t total = b_row + 2 * b_col + (sd ? b_row + 2 * b_col : b_col);
     void *arena = nullptr;
-    SG_TRY_CUDA(ctx, cudaMalloc(&arena, total));
+    SG_TRY_CUDA(ctx, arena_alloc(ctx, &arena, total));
     char *p = (char *)arena;
     auto carve = [&](size_t bytes) {
         uint32_t *q = (uint32_t *)p;
@@ -1264,10 +1278,10 @@ sg_status symmetric_weighted_csc(sg_ctx *ctx, sg_graph *g) {
     if (e == cudaSuccess && ne) e = cudaMemcpyAsync(cw, tw, 4ull * ne, cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
-        cudaFree(arena);
+        arena_free(ctx, arena, total);
         return cuda_status(ctx, e, "graph relayout");
     }
-    cudaFree(g->arena);
+    arena_free(ctx, g->arena, g->arena_bytes);
     g->arena = arena;
     g->arena_bytes = total;
     g->row = row;

@@ -45,3 +45,9 @@ sg_status device_transpose(sg_ctx *ctx, uint32_t nv, uint64_t ne, const uint32_t
 sg_status symmetric_weighted_csc(sg_ctx *ctx, sg_graph *g);
 
 }  // namespace sgb
+
+// For the tests of graph construction with little memory: builds on ctx go by
+// counting, allocations that would take the context's scratch and graph arrays
+// past `limit` bytes (0 = none) are refused, and *peak gets the most bytes held
+// since the call before.
+extern "C" sg_status sg_debug_build_memory(sg_ctx *ctx, int counting, uint64_t limit, uint64_t *peak);

@@ -23,6 +23,22 @@
 
 namespace sgb {
 struct Workspace;
+// Device bytes of a context: scratch and graph arrays.  `limit` refuses allocations past it as the
+// device does when it has no room: the tests' way to the paths for that case.
+struct MemUse {
+    size_t limit = ~size_t(0), used = 0, peak = 0;
+    bool fits(size_t bytes) const { return bytes <= limit && used <= limit - bytes; }
+    void add(size_t bytes) {
+        used += bytes;
+        peak = std::max(peak, used);
+    }
+};
+// Buffers gb_<prefix>_0 .. n - 1 of the graph workspace are in use by a build.
+struct BuildBuffers {
+    const char *prefix;
+    unsigned n = 0;
+    std::string name(unsigned k) const { return std::string("gb_") + prefix + "_" + std::to_string(k); }
+};
 }
 
 struct sg_ctx {
@@ -43,6 +59,9 @@ struct sg_ctx {
     // (between half its size and its size): reloading a graph costs no cudaMalloc/cudaFree
     void *spare_arena = nullptr;
     size_t spare_bytes = 0;
+    sgb::MemUse mem;
+    std::vector<const sgb::BuildBuffers *> building;  // of the build at hand, outermost first
+    bool build_by_counting = false;  // graph builds skip the radix sort (sg_debug_build_memory)
     bool persist_ref = false;  // holds a reference on the device's persisting-L2 set-aside
     // Contexts whose persistent launches run side by side on the device (a
     // server's slots): each launch takes at most 1/resident_share of a kernel's
@@ -94,18 +113,40 @@ struct Workspace {
     std::map<std::string, DevBuf> bufs;
     const cudaStream_t *stream = nullptr;  // the owning context's current stream
     cudaMemPool_t pool = nullptr;
+    MemUse *use = nullptr;
     Workspace() = default;
-    Workspace(const cudaStream_t *s, cudaMemPool_t p) : stream(s), pool(p) {}
+    explicit Workspace(sg_ctx *ctx) : stream(&ctx->stream), pool(device_pool(ctx->device)), use(&ctx->mem) {}
     Workspace(const Workspace &) = delete;
     Workspace &operator=(const Workspace &) = delete;
     bool ordered() const { return stream && pool; }
     ~Workspace() {
-        for (auto &kv : bufs)
-            if (kv.second.p) {
-                if (ordered()) cudaFreeAsync(kv.second.p, *stream);
-                else cudaFree(kv.second.p);
-            }
+        for (auto &kv : bufs) release(kv.second);
         if (ordered()) cudaStreamSynchronize(*stream);
+    }
+    void release(DevBuf &b) {
+        if (b.p) {
+            if (ordered()) cudaFreeAsync(b.p, *stream);
+            else cudaFree(b.p);
+            if (use) use->used -= b.bytes;
+        }
+        b = DevBuf{};
+    }
+    cudaError_t allocate(DevBuf &b, size_t bytes) {
+        if (use && !use->fits(bytes)) return cudaErrorMemoryAllocation;
+        cudaError_t e = ordered() ? cudaMallocFromPoolAsync(&b.p, bytes, pool, *stream) : cudaMalloc(&b.p, bytes);
+        if (e == cudaErrorMemoryAllocation && ordered()) {  // what the pool holds in other sizes goes back first
+            cudaGetLastError();
+            cudaStreamSynchronize(*stream);
+            cudaMemPoolTrimTo(pool, 0);
+            e = cudaMallocFromPoolAsync(&b.p, bytes, pool, *stream);
+        }
+        if (e != cudaSuccess) {
+            b.p = nullptr;
+            return e;
+        }
+        b.bytes = bytes;
+        if (use) use->add(bytes);
+        return cudaSuccess;
     }
     template <typename T>
     cudaError_t get(const char *name, size_t count, T **out, bool zero_new = false) {
@@ -114,15 +155,9 @@ struct Workspace {
         if (bytes == 0) bytes = 256;
         bytes = (bytes + 255) & ~size_t(255);
         if (b.bytes < bytes) {
-            if (b.p) {
-                if (ordered()) cudaFreeAsync(b.p, *stream);
-                else cudaFree(b.p);
-            }
-            b.p = nullptr;
-            b.bytes = 0;
-            cudaError_t e = ordered() ? cudaMallocFromPoolAsync(&b.p, bytes, pool, *stream) : cudaMalloc(&b.p, bytes);
+            release(b);
+            cudaError_t e = allocate(b, bytes);
             if (e != cudaSuccess) return e;
-            b.bytes = bytes;
             if (zero_new) {
                 e = ordered() ? cudaMemsetAsync(b.p, 0, bytes, *stream) : cudaMemset(b.p, 0, bytes);
                 if (e != cudaSuccess) return e;
@@ -131,14 +166,12 @@ struct Workspace {
         *out = (T *)b.p;
         return cudaSuccess;
     }
-    // Releases the buffers whose names start with `prefix`.
-    void drop(const char *prefix) {
+    // Releases the buffers whose names `which` accepts.
+    template <typename Which>
+    void drop(Which &&which) {
         for (auto it = bufs.begin(); it != bufs.end();) {
-            if (it->first.compare(0, std::strlen(prefix), prefix) == 0) {
-                if (it->second.p) {
-                    if (ordered()) cudaFreeAsync(it->second.p, *stream);
-                    else cudaFree(it->second.p);
-                }
+            if (which(it->first)) {
+                release(it->second);
                 it = bufs.erase(it);
             } else {
                 ++it;
@@ -170,9 +203,52 @@ namespace sgb {
 // Scratch of single-query calls on g: the context's, grow-only and shared by
 // all its graphs (work of a context is ordered on its stream), so creating
 // another graph allocates no new scratch.
-inline Workspace &graph_ws(sg_graph *g) {
-    if (!g->ctx->graph_ws) g->ctx->graph_ws = new Workspace(&g->ctx->stream, device_pool(g->ctx->device));
-    return *g->ctx->graph_ws;
+inline Workspace &graph_ws(sg_ctx *ctx) {
+    if (!ctx->graph_ws) ctx->graph_ws = new Workspace(ctx);
+    return *ctx->graph_ws;
+}
+inline Workspace &graph_ws(sg_graph *g) { return graph_ws(g->ctx); }
+
+inline void arena_free(sg_ctx *ctx, void *p, size_t bytes) {
+    if (!p) return;
+    cudaFree(p);
+    ctx->mem.used -= bytes;
+}
+inline void release_spare(sg_ctx *ctx) {
+    arena_free(ctx, ctx->spare_arena, ctx->spare_bytes);
+    ctx->spare_arena = nullptr;
+    ctx->spare_bytes = 0;
+}
+
+// Gives back what a context keeps from graph builds and no running step of one
+// uses: scratch (the radix sort's among it: not to be called inside a sort), the
+// spare arena and the pool's unused memory.
+inline void release_build_scratch(sg_ctx *ctx) {
+    cudaGetLastError();
+    auto unused = [&](const std::string &name) {
+        if (name.compare(0, 3, "gb_") != 0 || name == "gb_scan_parts") return false;
+        for (const BuildBuffers *b : ctx->building)
+            for (unsigned k = 0; k < b->n; ++k)
+                if (name == b->name(k)) return false;
+        return true;
+    };
+    if (ctx->graph_ws) ctx->graph_ws->drop(unused);
+    cudaStreamSynchronize(ctx->stream);
+    release_spare(ctx);
+    if (cudaMemPool_t pool = device_pool(ctx->device)) cudaMemPoolTrimTo(pool, 0);
+}
+
+// The memory of a graph's arrays; when the device has no room, once more
+// without the scratch of the build that made them.
+inline cudaError_t arena_alloc(sg_ctx *ctx, void **p, size_t bytes) {
+    auto once = [&] { return ctx->mem.fits(bytes) ? cudaMalloc(p, bytes) : cudaErrorMemoryAllocation; };
+    cudaError_t e = once();
+    if (e == cudaErrorMemoryAllocation) {
+        release_build_scratch(ctx);
+        e = once();
+    }
+    if (e == cudaSuccess) ctx->mem.add(bytes);
+    return e;
 }
 }  // namespace sgb
 

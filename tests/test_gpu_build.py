@@ -2,6 +2,7 @@
 sg_graph_create) against the reference converter's golden output, the oracle
 restatements of gtools and csr_tocsc, and, at full size, against the host
 generators (a shuffled raw edge stream must rebuild the same CSR)."""
+import ctypes
 import glob
 import os
 
@@ -26,6 +27,13 @@ def ctx():
 def _load(path):
     z = np.load(path)
     return {k: z[k] for k in z.files}
+
+
+def _debug(c, counting=False, limit=0):
+    """Path and memory of the context's graph builds; returns the most bytes held since the call before."""
+    peak = ctypes.c_uint64()
+    assert sg.load().sg_debug_build_memory(c._c, int(counting), ctypes.c_uint64(limit), ctypes.byref(peak)) == 0
+    return peak.value
 
 
 def _rows_of(off):
@@ -264,3 +272,62 @@ def test_released_arena_is_reused(ctx):
         G.close()
     finally:
         c.close()
+
+
+def _case(code, m=50000, nv=3000):
+    r = np.random.default_rng(code)
+    s, d = r.integers(0, nv, m).astype(np.uint32), r.integers(0, nv, m).astype(np.uint32)
+    s[: m // 4] = 7  # one long row
+    w = r.integers(0, 2**32, m, dtype=np.uint64).astype(np.uint32)
+    kw = dict(deself_cycle=bool(code & 1), deduplicate=bool(code & 2), d2ud=bool(code & 4), sort_rows=bool(code & 8))
+    return nv, s, d, w, kw
+
+
+def _check_built(G, want):
+    off, idx, w = G.copy_out()
+    assert all(np.array_equal(x, y) for x, y in zip((off, idx, w), want))
+    t = oracle.csr_tocsc(off, idx, w)
+    assert all(np.array_equal(x, y) for x, y in zip(G.copy_out(csc=True), t))
+
+
+@pytest.mark.parametrize("code", range(16))
+@pytest.mark.parametrize("nv,m", [(1, 5), (3000, 50000), (200, 4097), (70000, 3)])
+def test_build_by_counting(code, nv, m):
+    nv, s, d, w, kw = _case(code, m, nv)
+    c = sg.Context(0)
+    _debug(c, counting=True)
+    _check_built(c.build_graph(nv, s % nv, d, w, **kw), oracle.gtools_build(nv, s % nv, d, w, **kw))
+    c.close()
+
+
+@pytest.mark.parametrize("code", [0, 2, 5, 11])
+def test_build_with_little_memory(code):
+    """Whatever the radix sort lacks, its scratch, its output or the graph's own arrays, a build succeeds wherever
+    counting alone has room, also on a context that holds the scratch of earlier builds."""
+    nv, s, d, w, kw = _case(code)
+    want = oracle.gtools_build(nv, s, d, w, **kw)
+    peak = {}
+    for counting in (True, False):
+        c = sg.Context(0)
+        _debug(c, counting)
+        for _ in range(2):
+            c.build_graph(nv, s, d, w, **kw).close()
+        peak[counting] = _debug(c)
+        c.close()
+    assert peak[True] < peak[False]
+    for limit in np.linspace(peak[True], peak[False], 24).astype(int):
+        c = sg.Context(0)
+        _debug(c, limit=int(limit))
+        for _ in range(2):
+            G = c.build_graph(nv, s, d, w, **kw)
+            _check_built(G, want)
+            G.close()
+        assert _debug(c) <= limit
+        c.close()
+    c = sg.Context(0)  # and what does not fit is still refused
+    _debug(c, limit=peak[True] // 2)
+    with pytest.raises(sg.SGError):
+        c.build_graph(nv, s, d, w, **kw)
+    _debug(c)
+    _check_built(c.build_graph(nv, s, d, w, **kw), want)
+    c.close()
