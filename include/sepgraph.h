@@ -18,7 +18,7 @@
  *  - One sg_ctx per host thread.  All work of a context is ordered on its
  *    stream (sg_ctx_set_stream to share a caller's stream).
  *  - Indices are uint32 (index_t in include/groute/graphs/common.h:36);
- *    edge counts are uint64 at the boundary and must be < 2^32 inside.
+ *    edge counts are uint64 at the boundary and at most 2^32 - 1024 inside.
  */
 #ifndef SEPGRAPH_B200_H
 #define SEPGRAPH_B200_H

@@ -266,6 +266,9 @@ namespace sgb {
 // view from the device transpose: no host loop over the edges.
 sg_status create_graph(sg_ctx *ctx, uint32_t nv, uint64_t ne, const uint32_t *offsets, const uint32_t *indices,
                        const uint32_t *weights, uint32_t flags, sg_graph **out) {
+    if (ne > kMaxEdges)
+        return set_error(ctx, SG_ERR_INVALID_ARG, "edge count %llu exceeds the limit of %llu", (unsigned long long)ne,
+                         (unsigned long long)kMaxEdges);
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
     const bool has_csc = !(flags & SG_GRAPH_NO_CSC), symmetric = (flags & SG_GRAPH_SYMMETRIC) != 0;
     const bool full_csc = has_csc && !symmetric;
@@ -360,7 +363,6 @@ extern "C" {
 sg_status sg_graph_create(sg_ctx *ctx, uint32_t nv, uint64_t ne, const uint32_t *offsets, const uint32_t *indices,
                           const uint32_t *weights, uint32_t flags, sg_graph **out) {
     if (!ctx || !out || !offsets || (ne && !indices) || nv == 0) return SG_ERR_INVALID_ARG;
-    if (ne >= (1ull << 32)) return set_error(ctx, SG_ERR_INVALID_ARG, "edge count %llu exceeds uint32", (unsigned long long)ne);
     *out = nullptr;
     DeviceGuard dg(ctx->device);
     return sgb::create_graph(ctx, nv, ne, offsets, indices, weights, flags, out);

@@ -32,6 +32,10 @@ void graph_view_destroy(sg_graph *view);
 // resident blocks per SM (1, the default, lets a launch fill the device).
 void set_resident_share(sg_ctx *ctx, uint32_t share);
 
+// Most edges of a graph.  Edge indices are 32 bits, and the kernels step them
+// past a list's or the array's end by up to 512 before they compare.
+constexpr uint64_t kMaxEdges = (1ull << 32) - 1024;
+
 // Device graph from a CSR (host or device arrays): one upload, validation on
 // the device, and the in-edge (CSC) view from the device transpose.
 sg_status create_graph(sg_ctx *ctx, uint32_t nv, uint64_t ne, const uint32_t *offsets, const uint32_t *indices,

@@ -331,3 +331,11 @@ def test_build_with_little_memory(code):
     _debug(c)
     _check_built(c.build_graph(nv, s, d, w, **kw), want)
     c.close()
+
+
+@pytest.mark.parametrize("ne", [2**32 - 1023, 2**32 - 1, 2**32])
+def test_edge_counts_near_the_index_range_are_refused(ctx, ne):
+    """Before the arrays are looked at: these hold one vertex and no edge."""
+    off, idx = np.zeros(2, np.uint32), np.zeros(1, np.uint32)
+    with pytest.raises(sg.SGError, match="INVALID_ARG"):
+        ctx.graph_from_csr(off.ctypes.data, idx.ctypes.data, nv=1, ne=ne)
