@@ -149,24 +149,26 @@ sg_graph *sg_server::view(int slot, uint32_t graph_id) {
 uint64_t sg_server::estimate(const std::vector<Pending> &b) const {
     // Device scratch of one batch: per-team workspaces sized for the largest
     // graph (about 32 bytes per vertex, 64 with BC's path counts, level stack,
-    // dependencies and records; at most one team per query and per resident block),
-    // multi-source BFS masks and level rows, and staging for host outputs.
+    // dependencies and records, and 0.11 per edge for the pull rounds' tiles and
+    // chunks; at most one team per query and per resident block), multi-source BFS
+    // masks, queues, level planes and level rows, and staging for host outputs.
     if (b.empty()) return 0;
     const int algo = b.front().q.algo;
-    uint64_t nv_max = 0, outs = 0;
+    uint64_t nv_max = 0, ne_max = 0, outs = 0;
     std::map<uint32_t, uint64_t> per_graph;
     for (auto &p : b) {
         const uint64_t nv = graphs[p.q.graph_id].nv;
         nv_max = std::max(nv_max, nv);
+        ne_max = std::max(ne_max, graphs[p.q.graph_id].ne);
         outs += 8 * nv;
         per_graph[p.q.graph_id]++;
     }
     const uint64_t teams = std::min<uint64_t>(b.size(), 148ull * 8);
-    uint64_t bytes = teams * nv_max * (algo == SG_QUERY_BC ? 64 : 32) + outs;
+    uint64_t bytes = teams * (nv_max * (algo == SG_QUERY_BC ? 64 : 32) + ne_max / 9) + outs;
     if (algo == SG_QUERY_BFS)
         for (auto &kv : per_graph)
             if (kv.second >= std::max(1u, cfg.msbfs_min))
-                bytes += graphs[kv.first].nv * (32 + 4 * std::min<uint64_t>(kv.second, 64));
+                bytes += graphs[kv.first].nv * (32 + 12 + 40 + 4 * std::min<uint64_t>(kv.second, 64));
     if (algo == SG_QUERY_BC)  // multi-source BC scratch: 32 path counts, dependencies, q, masks, lists, rows
         for (auto &kv : per_graph)
             if (kv.second >= std::max(1u, cfg.msbfs_min)) bytes += graphs[kv.first].nv * 1000ull;

@@ -208,3 +208,25 @@ def test_bc_groups_match_alone():
             assert np.allclose(got, want, rtol=1e-4, atol=1e-5), (g, s)
     finally:
         ctx.close()
+
+
+def test_batch_estimates_cover_multi_source_bfs(setup, tmp_path, monkeypatch):
+    """Masks, queues, level planes and one level row per source of every batch that goes multi-source."""
+    ctx, graphs = setup
+    log = tmp_path / "batches.log"
+    monkeypatch.setenv("SEPGRAPH_SERVER_LOG", str(log))
+    h, G = graphs[3]  # dense: the kernel with level planes
+    srv = sg.Server(0, max_batch=64)
+    gid = srv.add_graph(G)
+    outs = [np.empty(h.nv, np.uint32) for _ in range(128)]
+    for k, o in enumerate(outs):
+        srv.submit("bfs", gid, int(h.pick_sources(1, k)[0]), o)
+    srv.drain()
+    srv.close()
+    lines = [line.split() for line in log.read_text().splitlines()]
+    sizes = [(int(x[5]), int(x[7])) for x in lines]
+    assert sum(q for q, _ in sizes) == 128 and max(q for q, _ in sizes) >= 8
+    for q, est in sizes:
+        if q >= 8:
+            team_scratch, staging = 32 * q, 8 * q
+            assert est >= h.nv * (team_scratch + staging + 32 + 12 + 40 + 4 * min(q, 64))
