@@ -969,6 +969,7 @@ sg_status prepare_batch(sg_ctx *ctx, sgb::Workspace &ws, std::vector<engine::Bat
             if (p.forced == V_ASYNC_PUSH_DD) {
                 B.kernel = (const void *)batched_engine_kernel<App, TV, TB, TW, V_ASYNC_PUSH_DD>;
                 which = 1;
+                p.collect = 0;  // that kernel keeps no statistics (a graph without in-edges forces the push late)
             }
     }
     int max_bps = 0;

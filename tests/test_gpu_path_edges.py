@@ -194,6 +194,23 @@ def test_bc_above_the_dense_size(ctx, variant):
     G.close()
 
 
+def test_default_sssp_batch_without_in_edges(ctx):
+    """A graph without in-edges makes the whole batch push, hub chunks included."""
+    queries, wants = [], []
+    for k, no_csc in ((700, True), (2000, False)):
+        nv, s, d = _hub(k)
+        off, idx, w = _csr(nv, np.concatenate([s, d]), np.concatenate([d, s]),
+                           np.random.default_rng(k).integers(1, 64, 2 * len(s)).astype(np.uint32))
+        G = ctx.graph_from_csr(off, idx, w, no_csc=no_csc)
+        for src in (0, nv - 1, 5):
+            queries.append((G, src))
+            wants.append(oracle.sssp(off, idx, w, src))
+    outs = ctx.sssp_batch(queries, max_iteration=100000)[0]
+    assert all(np.array_equal(x, y) for x, y in zip(outs, wants))
+    for G in {id(g): g for g, _ in queries}.values():
+        G.close()
+
+
 def _gap(nv, m, at, gap, seed):
     """A random graph whose ids from `at` on are moved up by `gap` unused ones."""
     s, d = _random(nv, m, seed)
