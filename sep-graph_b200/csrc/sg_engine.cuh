@@ -296,7 +296,7 @@ struct Acc {
     uint32_t heavy_hi, heavy_lo;
     unsigned long long edges;
     uint32_t active;
-    uint32_t push_hi, push_lo;  // bits set in a bitmap worklist / the far pile (or left in it)
+    uint32_t push_hi, push_lo;  // bits set in a bitmap worklist / the far pile (or left in it, see exact_far)
     uint32_t popped;
     // This warp's staged appends to the near worklist (push rounds without
     // lookahead): kStageItems entries, the first stage_n filled (the same in
@@ -757,10 +757,7 @@ struct EngineKernel {
         }
         bool w_hi = want && hi;
         const bool w_lo = want && !hi;
-        if (w_lo) {  // the far pile is a bitmap (see push_far)
-            dev::bitmap_set_nr(a.qflag[s.qlo], dst);
-            ++acc.push_lo;
-        }
+        if (w_lo) set_far(a, acc, s, dst);
         if (a.p.bitmap_frontier) {
             // no dedupe round trip and no append: the bit is the worklist entry
             if (w_hi) {
@@ -777,7 +774,23 @@ struct EngineKernel {
                 __syncwarp();
             }
         }
-        if (w_hi || w_lo) count_enq(a, acc, w_hi, dst);
+        if (w_hi) count_enq(a, acc, true, dst);
+    }
+
+    // Traced runs report the far pile's size and out-edges: there its count
+    // follows every bit set and cleared, where others only need to know whether
+    // it is empty.
+    static __device__ __forceinline__ bool exact_far(const Args &a) { return kCollect && a.p.collect; }
+
+    // The far pile is a bitmap (see push_far): the bit is the entry.
+    static __device__ __forceinline__ void set_far(const Args &a, Acc &acc, const Snap &s, uint32_t dst) {
+        if (exact_far(a)) {
+            if (!dev::bitmap_set(a.qflag[s.qlo], dst)) return;
+        } else {
+            dev::bitmap_set_nr(a.qflag[s.qlo], dst);
+        }
+        ++acc.push_lo;
+        count_enq(a, acc, false, dst);
     }
 
     static __device__ __forceinline__ void put(const Args &a, Acc &acc, uint32_t slot, bool staged, uint32_t pos,
@@ -834,11 +847,7 @@ struct EngineKernel {
 #pragma unroll
         for (int j = 0; j < K; ++j) {
             w[j] = want[j] && hi[j];
-            if (want[j] && !hi[j]) {  // far pile: the bit is the entry
-                dev::bitmap_set_nr(a.qflag[s.qlo], dst[j]);
-                count_enq(a, acc, false, dst[j]);
-                ++acc.push_lo;
-            }
+            if (want[j] && !hi[j]) set_far(a, acc, s, dst[j]);
         }
         if (a.p.bitmap_frontier) {
 #pragma unroll
@@ -882,10 +891,8 @@ struct EngineKernel {
                 return;
             }
         }
-        if (!hi) {  // far pile: the bit is the entry
-            dev::bitmap_set_nr(a.qflag[s.qlo], dst);
-            ++acc.push_lo;
-            count_enq(a, acc, false, dst);
+        if (!hi) {
+            set_far(a, acc, s, dst);
             return;
         }
         if (!dev::bitmap_set(a.qflag[s.qhi], dst)) return;
@@ -1652,6 +1659,10 @@ struct EngineKernel {
                         dev::bitmap_and_nr(bits + wi, ~gone);
                     }
                 }
+                if (exact_far(a))
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (in[q]) acc.scout_lo -= out_degree(a, v[q]);
                 if constexpr (!has_min_relax<App, TB, TW>::value) __threadfence();
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
@@ -1673,7 +1684,7 @@ struct EngineKernel {
             popped += __popc(gone);
         }
         if (n) push_item(app, a, s, w, true, lb, acc, lq, lane < n ? buf[lane] : 0u, lane < n, false);
-        acc.push_lo += kept;
+        acc.push_lo += exact_far(a) ? 0u - popped : kept;
         acc.popped += popped;
     }
 
@@ -1784,7 +1795,8 @@ struct EngineKernel {
     // an atomic on one counter.  `sync` writes the combined buffer to
     // tmp (SYNC_PULL_*), else back into buffer (ASYNC_PULL_DD, algo_variants.cuh:842-849).
     // With `split`, scheduled vertices above kPullSplit in-edges list their chunks.
-    static __device__ void combine_all(App &app, const Args &a, bool sync, bool build_middle, bool split, Acc &acc) {
+    static __device__ void combine_all(App &app, const Args &a, bool dd, bool sync, bool build_middle, bool split,
+                                       Acc &acc) {
         const uint32_t lane = dev::lane_id();
         const uint32_t N = a.csr.nnodes;
         bool all = true;
@@ -1840,7 +1852,7 @@ struct EngineKernel {
                     if (k > 0 && !several) break;
                     const uint64_t w = w0 + (uint64_t)k * nwarps();
                     const uint64_t v = w * 32 + lane;
-                    if (split && want[k]) list_pull_chunks(a, (uint32_t)v, beg[k], end[k] - beg[k], acc);
+                    if (split && want[k]) list_pull_chunks(a, (uint32_t)v, beg[k], end[k] - beg[k], dd, acc);
                     const uint32_t m = __ballot_sync(dev::kFullMask, want[k]);
                     if (lane == 0 && w * 32 < N) a.middle[w] = m;
                     all = all && __all_sync(dev::kFullMask, want[k] || v >= N);
@@ -1858,7 +1870,7 @@ struct EngineKernel {
                         a.buffer[v] = pr.first;
                     want = pr.second;
                     if (want && split)
-                        list_pull_chunks(a, v, a.csc.begin_edge(v), a.csc.end_edge(v) - a.csc.begin_edge(v), acc);
+                        list_pull_chunks(a, v, a.csc.begin_edge(v), a.csc.end_edge(v) - a.csc.begin_edge(v), dd, acc);
                 }
                 if (build_middle) {
                     const uint32_t m = __ballot_sync(dev::kFullMask, want);
@@ -1871,8 +1883,9 @@ struct EngineKernel {
     }
 
     static __device__ __forceinline__ void list_pull_chunks(const Args &a, uint32_t v, uint32_t beg, uint32_t deg,
-                                                            Acc &acc) {
-        if (has_pull_term<App>::value) acc.active += deg;  // in-edges this round scans
+                                                            bool dd, Acc &acc) {
+        // in-edges this round scans (a topology-driven round counts its active vertices there)
+        if (has_pull_term<App>::value && dd) acc.active += deg;
         if (deg <= kPullSplit) return;
         Counters *n = &a.ctrl->cnt;
         const uint32_t nch = (deg + kPullChunk - 1) / kPullChunk;
@@ -2874,9 +2887,7 @@ struct EngineKernel {
             // (driver.cuh:668-675), whose slot stays where it is
             rs.prio_raw = to_raw<TB>((TB)(from_raw<TB>(rs.prio_raw) + from_raw<TB>(a.p.prio_step_raw)));
             rs.pile = 1;
-            n->qcount[rs.qlo] = 0;
-            n->scout[rs.qlo] = 0;
-            n->heavy_enq[rs.qlo] = 0;
+            if (!a.p.collect) n->qcount[rs.qlo] = 0;  // push_far counts what stays, see exact_far
         }
         const uint32_t consumed = rs.qin;
         rs.qin = rs.qhi;
@@ -2917,7 +2928,8 @@ struct EngineKernel {
             n->heavy_count[cur] = 0;
             n->chunk_count[cur] = 0;
         }
-        pre_bookkeeping(a, ps, rs.F, sc[rs.qin]);
+        if (rs.pile) pre_bookkeeping(a, ps, qc[rs.qlo], sc[rs.qlo]);
+        else pre_bookkeeping(a, ps, rs.F, sc[rs.qin]);
         publish(a, ps);
         ps.t_round_start = dev::globaltimer_ns();
     }
@@ -3122,7 +3134,7 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
                     K::compute_tile_rows(a);
                     tiles_listed = true;
                 }
-                K::combine_all(app, a, sync, !reduce_td, !reduce_td && a.pull_chunks && lb_pull != LB_NONE, acc);
+                K::combine_all(app, a, dd, sync, !reduce_td, !reduce_td && a.pull_chunks && lb_pull != LB_NONE, acc);
                 if (term_tiles) K::flush_acc(a, acc, s.qhi, s.qlo);  // the in-edges to scan
                 if (!grid_sync(c, tmo, nop)) return false;
                 if (tiles && dev::ld_l2(&c->cnt.middle_count) == 0) {

@@ -211,6 +211,64 @@ def test_default_sssp_batch_without_in_edges(ctx):
         G.close()
 
 
+def _near_far_rounds(nv, off, idx, w, src, delta):
+    """(in_nodes, out_nodes, in_workload, out_workload) of every near/far round on a tree, where each vertex gets its
+    distance once and the rounds do not depend on the order of the work."""
+    deg = np.diff(off.astype(np.int64))
+    dist = {src: 0}
+    near, far, limit, rounds, pile = [src], set(), delta, [], False
+    work = lambda vs: int(sum(deg[v] for v in vs))
+    while near or far:
+        if pile:
+            take = [v for v in far if dist[v] < limit]
+            n_in, w_in = len(far), work(far)
+            far -= set(take)
+        else:
+            take, n_in, w_in = near, len(near), work(near)
+        near = []
+        for u in take:
+            for e in range(off[u], off[u + 1]):
+                v = int(idx[e])
+                dist[v] = dist[u] + int(w[e])
+                if dist[v] < limit:
+                    near.append(v)
+                else:
+                    far.add(v)
+        rounds.append((n_in, len(near) + len(far), w_in, work(near) + work(far)))
+        pile = not near
+        if pile:
+            limit += delta
+    return rounds
+
+
+@pytest.mark.parametrize("lb", ["fine", "none"])
+@pytest.mark.parametrize("fan,nv", [(3, 4000), (12, 9000)])
+def test_trace_of_near_far_rounds(ctx, lb, fan, nv):
+    child = np.arange(1, nv, dtype=np.uint32)
+    off, idx, w = _csr(nv, (child - 1) // fan, child, np.random.default_rng(fan).integers(1, 50, nv - 1).astype(np.uint32))
+    G = ctx.graph_from_csr(off, idx, w)
+    dist, st, tr = G.sssp(0, variant="async_push_dd", priority="low_high", priority_delta=20, lb_push=lb,
+                          max_iteration=100000, trace_capacity=4096)
+    assert np.array_equal(dist, oracle.sssp(off, idx, w, 0))
+    want = _near_far_rounds(nv, off, idx, w, 0, 20)
+    got = [(t["in_nodes"], t["out_nodes"], t["in_workload"], t["out_workload"]) for t in tr]
+    assert got == want
+    G.close()
+
+
+def test_trace_of_topology_driven_bc_pull(ctx):
+    """out_nodes of a topology-driven round = the vertices that are active after it: those with a level so far (and in
+    the first round the source once more, active at the start)."""
+    nv, s, d = _hub(700)
+    off, idx, _ = _csr(nv, s, d)
+    level = oracle.bfs(off, idx, 0)
+    G = ctx.graph_from_csr(off, idx)
+    bc, sigma, st = G.bc(0, variant="sync_pull_td", max_iteration=6, trace_capacity=64)
+    assert st.n_trace == 6
+    assert [st.trace[r].out_nodes for r in range(6)] == [int((level <= r + 1).sum()) + (r == 0) for r in range(6)]
+    G.close()
+
+
 def _gap(nv, m, at, gap, seed):
     """A random graph whose ids from `at` on are moved up by `gap` unused ones."""
     s, d = _random(nv, m, seed)
