@@ -394,6 +394,19 @@ struct has_min_relax<App, TB, TW,
                          std::declval<uint32_t>(), std::declval<uint32_t>(), std::declval<TW>(), std::declval<TB>()))>>
     : std::integral_constant<bool, std::is_same<TB, uint32_t>::value> {};
 
+// An extension that stands for a method of the functor (CombinePull for
+// CombineValueBuffer, say) holds for the method of the class that declares it
+// or of a base: a derived functor that overrides the method alone gets its
+// override, not the inherited extension.
+template <typename C, typename R, typename... A>
+C declarer(R (C::*)(A...));
+template <typename C, typename R, typename... A>
+C declarer(R (C::*)(A...) const);
+template <typename C, typename TB>  // the unweighted one of the two overloads
+C accumulate_declarer(int (C::*)(uint32_t, uint32_t, TB *, TB));
+template <typename Extension, typename Method>
+struct stands_for : std::is_base_of<Method, Extension> {};
+
 // Optional functor extension (no reference counterpart): a functor whose
 // frontier sources of one data-driven pull round all offer the same value, and
 // whose AccumulateBuffer adds a term of the source and never breaks, declares
@@ -406,7 +419,7 @@ template <typename App, typename = void>
 struct has_pull_term : std::false_type {};
 template <typename App>
 struct has_pull_term<App, std::void_t<decltype(std::declval<const App &>().PullTerm(std::declval<uint32_t>()))>>
-    : std::true_type {};
+    : stands_for<decltype(declarer(&App::PullTerm)), decltype(accumulate_declarer(&App::AccumulateBuffer))> {};
 
 // Optional functor extension (no reference counterpart): a PullReduce functor
 // whose vertices need scheduling exactly when IsActiveNode(buffer) holds after
@@ -417,7 +430,10 @@ template <typename App, typename = void>
 struct has_active_is_pending : std::false_type {};
 template <typename App>
 struct has_active_is_pending<App, std::void_t<decltype(std::declval<const App &>().ActiveIsPending())>>
-    : std::true_type {};
+    : std::bool_constant<
+          stands_for<decltype(declarer(&App::ActiveIsPending)), decltype(declarer(&App::IsActiveNode))>::value &&
+          stands_for<decltype(declarer(&App::ActiveIsPending)),
+                     decltype(accumulate_declarer(&App::AccumulateBuffer))>::value> {};
 // A push round is dense when its worklist's out-edges are at least this share
 // (1 / kDenseShare) of all edges: a dense round costs a pass over all edges at
 // about twice the rate of the queued one.
@@ -440,7 +456,8 @@ template <typename App, typename = void>
 struct has_take_frontier : std::false_type {};
 template <typename App>
 struct has_take_frontier<App, std::void_t<decltype(std::declval<App &>().TakeFrontier(
-                                  std::declval<const uint32_t *>(), 0u, 0u, 0u))>> : std::true_type {};
+                                  std::declval<const uint32_t *>(), 0u, 0u, 0u))>>
+    : stands_for<decltype(declarer(&App::TakeFrontier)), decltype(declarer(&App::CombineValueBuffer))> {};
 
 // Optional functor extension (no reference counterpart): CombineValueBuffer of
 // a pull round on copies of the vertex's value and buffer,
@@ -452,8 +469,8 @@ struct has_combine_pull : std::false_type {};
 template <typename App, typename TV, typename TB>
 struct has_combine_pull<App, TV, TB,
                         std::void_t<decltype(std::declval<App &>().CombinePull(
-                            std::declval<uint32_t>(), std::declval<TV &>(), std::declval<TB &>()))>> : std::true_type {
-};
+                            std::declval<uint32_t>(), std::declval<TV &>(), std::declval<TB &>()))>>
+    : stands_for<decltype(declarer(&App::CombinePull)), decltype(declarer(&App::CombineValueBuffer))> {};
 
 // Edge range of chunk k of a heavy vertex's list [beg, beg + deg): chunks are
 // cut on the 4-edge grid (from beg rounded down to a multiple of 4) so that
