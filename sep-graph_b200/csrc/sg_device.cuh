@@ -60,9 +60,6 @@ __device__ __forceinline__ T ld_l2(const T *p) {
     return __ldcg(p);
 }
 
-// 16-byte read-only load (ld.global.nc.v4); p must be 16-byte aligned.
-__device__ __forceinline__ uint4 ldg_v4(const uint32_t *p) { return __ldg(reinterpret_cast<const uint4 *>(p)); }
-
 // Streamed graph arrays (edge destinations, weights, in-edge sources) are read
 // with an L2 evict-first cache policy: a traversal streams hundreds of MB of
 // them through L2 once, and without the hint they push out the vertex state

@@ -194,8 +194,9 @@ struct KArgs {
     // Edge-tiled pull (functors with PullReduce, unweighted, topology-driven;
     // min-relax functors): tile_row[t] = the in-edge row holding CSC edge
     // t * kPullTileEdges (ceil(E / kPullTileEdges) + 1 entries, the last = the
-    // row of the last edge), filled at the launch's start or in its first pull round; null =
-    // the destination-per-lane pull is used instead.
+    // row of the last edge), filled at the launch's start or in its first pull
+    // round.  Every launch whose rounds may be topology-driven pulls of a
+    // PullReduce functor has it; null = the others go over destinations.
     uint32_t *tile_row = nullptr;
     // Pull over destinations: (vertex, first in-edge, in-edges, -) chunks of
     // the round's vertices above kPullSplit in-edges, listed by its combine
@@ -257,9 +258,6 @@ struct WarpLB {
         };
     };
     __device__ __forceinline__ TBuffer *tile_values() { return reinterpret_cast<TBuffer *>(tile); }
-    // topology-driven pull without tiles: each lane's first and last (possibly shared) segment
-    __device__ __forceinline__ uint32_t *partk(int k) { return heavy_src + 32 * k; }
-    __device__ __forceinline__ TBuffer *part(int k) { return heavy_pay + 32 * k; }
     TBuffer pay[32];
     // push rounds: heavy vertices not registered yet (see stage_heavy)
     // (edge tiles keep the tile's values here, in edge order: no push runs then)
@@ -2290,94 +2288,6 @@ struct EngineKernel {
         count_enq(a, acc, true, v);
     }
 
-    // Topology-driven pull for functors with PullReduce: the warp walks the
-    // concatenated in-edge lists of 32 destinations (edge-balanced), folds the
-    // pulled values per destination in shared memory and issues one
-    // AccumulateBuffer per destination.  Destinations above heavy_threshold
-    // in-edges are split into chunks handled by pull_reduce_chunks.
-    static __device__ void pull_reduce_td(App &app, const Args &a, const Snap &s, WarpLB<TB> &w, Acc &acc) {
-        if constexpr (has_pull_reduce<App, TB>::value && std::is_same<TW, graphs::NoWeight>::value) {
-            const uint32_t lane = dev::lane_id();
-            const uint32_t N = a.csr.nnodes;
-            const TB *srcbuf = a.tmp;
-            for (uint32_t base = gwarp() * 32; base < N; base += nwarps() * 32) {
-                const uint32_t v = base + lane;
-                uint32_t beg = 0, deg = 0;
-                if (v < N) {
-                    beg = a.csc.begin_edge(v);
-                    deg = a.csc.end_edge(v) - beg;
-                }
-                const bool heavy = deg > a.p.heavy_threshold;
-                register_heavy(a, s.round & 1u, heavy, v, beg, deg, app.PullIdentity());
-                if (heavy) deg = 0;
-                const uint32_t incl = dev::warp_inclusive_scan(deg);
-                const uint32_t total = __shfl_sync(dev::kFullMask, incl, 31);
-                w.excl[lane] = incl - deg;
-                w.beg[lane] = beg;
-                w.pay[lane] = app.PullIdentity();
-                __syncwarp();
-                // Each lane reduces one contiguous 1/32 of the warp's concatenated
-                // in-edge lists, four independent gathers at a time, with one owner
-                // search at its start; a destination wholly inside one lane's range
-                // is written by that lane, the (at most two) segments a lane shares
-                // with neighbouring lanes are combined afterwards.
-                const uint32_t per = (total + 31) / 32;
-                const uint32_t lo = min(total, lane * per), hi = min(total, lo + per);
-                w.partk(0)[lane] = w.partk(1)[lane] = 0xffffffffu;
-                if (lo < hi) {
-                    uint32_t k = owner(w.excl, lo);
-                    uint32_t e = lo;
-                    bool first = true;
-                    while (e < hi) {
-                        const uint32_t seg_lo = w.excl[k];
-                        uint32_t seg_hi = total;  // next lane with a larger start
-                        for (uint32_t j = k + 1; j < 32; ++j)
-                            if (w.excl[j] > seg_lo) {
-                                seg_hi = w.excl[j];
-                                break;
-                            }
-                        const uint32_t end = min(hi, seg_hi);
-                        const uint32_t *src = a.csc.edge_source;
-                        const uint32_t off = w.beg[k] - seg_lo;  // CSC edge of e is off + e (mod 2^32)
-                        TB r = app.PullIdentity();
-                        for (; e + 4 <= end; e += 4) {
-                            const uint32_t s0 = __ldg(src + (off + e)), s1 = __ldg(src + (off + e + 1));
-                            const uint32_t s2 = __ldg(src + (off + e + 2)), s3 = __ldg(src + (off + e + 3));
-                            const TB g0 = dev::ld_l2(srcbuf + s0), g1 = dev::ld_l2(srcbuf + s1);
-                            const TB g2 = dev::ld_l2(srcbuf + s2), g3 = dev::ld_l2(srcbuf + s3);
-                            r = app.PullReduce(r, app.PullReduce(app.PullReduce(g0, g1), app.PullReduce(g2, g3)));
-                        }
-                        for (; e < end; ++e) r = app.PullReduce(r, dev::ld_l2(srcbuf + __ldg(src + (off + e))));
-                        const bool shared = seg_lo < lo || seg_hi > hi;  // other lanes hold part of k
-                        if (!shared) {
-                            w.pay[k] = r;
-                        } else {
-                            const int slot = first ? 0 : 1;
-                            w.partk(slot)[lane] = k;
-                            w.part(slot)[lane] = r;
-                        }
-                        first = false;
-                        // next destination with edges
-                        while (k < 31 && w.excl[k + 1] <= e) ++k;
-                    }
-                }
-                __syncwarp();
-                {
-                    TB r = w.pay[lane];
-                    for (uint32_t j = 0; j < 32; ++j) {
-                        if (w.partk(0)[j] == lane) r = app.PullReduce(r, w.part(0)[j]);
-                        if (w.partk(1)[j] == lane) r = app.PullReduce(r, w.part(1)[j]);
-                    }
-                    w.pay[lane] = r;
-                }
-                __syncwarp();
-                if (v < N && deg > 0) accumulate<App, TB, TW>(app, a.csc_w, v, v, beg, a.buffer + v, w.pay[lane]);
-                if (lane == 0) acc.edges += total;
-                __syncwarp();
-            }
-        }
-    }
-
     // Largest row r in [lo, hi] with col_start[r] <= e: the in-edge row that
     // holds CSC edge e (empty rows share their start with the next row, so the
     // largest such r is the non-empty one).
@@ -2668,36 +2578,6 @@ struct EngineKernel {
                     accumulate<App, TB, TW>(app, a.csc_w, r, r, 0, a.buffer + r, run);
                 }
                 if (lane == 0) acc.edges += t1;
-            }
-        }
-    }
-
-    static __device__ void pull_reduce_chunks(App &app, const Args &a, uint32_t set, Acc &acc) {
-        if constexpr (has_pull_reduce<App, TB>::value && std::is_same<TW, graphs::NoWeight>::value) {
-            const uint32_t C = min(dev::ld_l2(&a.ctrl->cnt.chunk_count[set]), a.chunk_cap);
-            const uint32_t H = min(dev::ld_l2(&a.ctrl->cnt.heavy_count[set]), a.heavy_cap);
-            const uint32_t *own = a.chunk_owner + (size_t)set * a.chunk_cap;
-            const HeavyItem<TB> *items = a.heavy + (size_t)set * a.heavy_cap;
-            const uint32_t lane = dev::lane_id();
-            const uint32_t ce = a.p.chunk_edges;
-            for (uint32_t ch = gwarp(); ch < C; ch += nwarps()) {
-                const uint32_t e = dev::ld_l2(own + ch);
-                if (e >= H) continue;
-                const HeavyItem<TB> h = items[e];
-                if (ch < h.chunk_base) continue;
-                uint32_t lo, hi;
-                chunk_span(h.beg, h.deg, ce, ch - h.chunk_base, &lo, &hi);
-                if (lo >= hi) continue;
-                const uint32_t len = hi - lo;
-                TB r = app.PullIdentity();
-                for (uint32_t k = lane; k < len; k += 32)
-                    r = app.PullReduce(r, dev::ld_l2(a.tmp + a.csc.edge_src(lo + k)));
-#pragma unroll
-                for (int d = 16; d > 0; d >>= 1) r = app.PullReduce(r, __shfl_xor_sync(dev::kFullMask, r, d));
-                if (lane == 0) {
-                    accumulate<App, TB, TW>(app, a.csc_w, h.src, h.src, h.beg, a.buffer + h.src, r);
-                    acc.edges += len;
-                }
             }
         }
     }
@@ -3158,13 +3038,8 @@ __device__ bool run_instance(const App &app_in, const KArgs<TV, TB, TW> &a) {
                     K::pull_tiles_relax(app, a, s, my_lb, dd, sync, acc, stage);
                 } else if (term_tiles && (uint64_t)dev::ld_l2(&c->cnt.active_count) * kTermShare >= a.csc.nedges) {
                     K::pull_tiles_terms(app, a, s, my_lb, sync, acc, stage);
-                } else if (reduce_td && a.tile_row) {
-                    K::pull_tiles(app, a, my_lb, acc);
                 } else if (reduce_td) {
-                    K::pull_reduce_td(app, a, s, my_lb, acc);
-                    K::flush_acc(a, acc, s.qhi, s.qlo);
-                    if (!grid_sync(c, tmo, nop)) return false;
-                    K::pull_reduce_chunks(app, a, set, acc);
+                    K::pull_tiles(app, a, my_lb, acc);
                 } else {
                     K::pull_phase(app, a, s, my_lb, dd, sync, lb_pull, acc, stage);
                 }

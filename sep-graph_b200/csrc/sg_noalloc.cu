@@ -60,7 +60,7 @@ constexpr uint32_t kChunkCap = kNoAllocMaxEdges / kChunkEdges + 2 * kHeavyCap + 
 constexpr size_t kOffBuffer = 0;
 constexpr size_t kOffTmp = kOffBuffer + align256(4ull * kNoAllocMaxVertices);
 constexpr size_t kOffQueue = kOffTmp + align256(4ull * kNoAllocMaxVertices);
-constexpr size_t kOffMiddle = kOffQueue + 3 * align256(4ull * kNoAllocMaxVertices);
+constexpr size_t kOffMiddle = kOffQueue + 2 * align256(4ull * kNoAllocMaxVertices);
 constexpr size_t kOffBitmap = kOffMiddle + align256(4ull * kNoAllocMaxVertices);
 constexpr size_t kOffFlag = kOffBitmap + 2 * align256(4ull * kWords);
 constexpr size_t kOffHeavy = kOffFlag + 3 * align256(4ull * kWords);
@@ -154,7 +154,7 @@ extern "C" sg_status sg_bfs_noalloc(const uint32_t *offsets, const uint32_t *ind
     a.value = levels_out;
     a.buffer = (uint32_t *)(base + kOffBuffer);
     a.tmp = (uint32_t *)(base + kOffTmp);
-    for (int k = 0; k < 3; ++k) a.queue[k] = (uint32_t *)(base + kOffQueue + k * align256(4ull * kNoAllocMaxVertices));
+    for (int k = 0; k < 2; ++k) a.queue[k] = (uint32_t *)(base + kOffQueue + k * align256(4ull * kNoAllocMaxVertices));
     a.queue_cap = nv;
     for (int k = 0; k < 2; ++k) a.bitmap[k] = (uint32_t *)(base + kOffBitmap + k * align256(4ull * kWords));
     for (int k = 0; k < 3; ++k) a.qflag[k] = (uint32_t *)(base + kOffFlag + k * align256(4ull * kWords));
