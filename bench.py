@@ -339,6 +339,21 @@ def cpu_baseline(h, srcs, budget_s=20.0):
             "seconds": t_tot, "results": results}
 
 
+def split_details(line):
+    """(the result line, its details): the autotuner's report and the extra sections are some 30 KB and go to stderr,
+    so that the line itself stays whole where only the end of stdout is kept.  The sections' parity flags are summed
+    up in the line."""
+    line = dict(line, tuning=dict(line["tuning"]), parity=dict(line["parity"]))
+    details = {"autotune_report": line["tuning"].pop("autotune_report", None), "extra": line.pop("extra", {})}
+    flags = {k: bool(v) for name, sec in details["extra"].items() for k, v in _parity_flags(sec, name)}
+    if flags:
+        line["parity"]["extra_checks"] = len(flags)
+        line["parity"]["extra_failed"] = sorted(k for k, v in flags.items() if not v)[:8]
+        line["parity"]["sections"] = {name: sec.get("bench_seconds") for name, sec in details["extra"].items()}
+    details["parity"] = flags
+    return line, details
+
+
 def run_reference(a):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
@@ -534,11 +549,9 @@ def run_ours(a):
         for k, (_, g) in list(cache.items()):
             if k != "rmat22":
                 g.close()
-    if "extra" in line:
-        for name, sec in line["extra"].items():
-            for k, v in _parity_flags(sec, name):
-                line["parity"][k] = v
     if rank == 0:
+        line, details = split_details(line)
+        print(json.dumps(details), file=sys.stderr, flush=True)
         print(json.dumps(line), flush=True)
     G.close()
     ctx.close()

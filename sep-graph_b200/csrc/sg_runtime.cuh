@@ -467,7 +467,10 @@ inline int resident_blocks_per_sm(const sg_ctx *ctx, int max_bps) {
 // graphs of 20,011 vertices (0.5 M edges) 0.76 / 0.77 / 0.91 / 1.01 / 1.02 ms, of
 // 100,003 (2.8 M) 1.49 / 1.29 / 1.16 / 1.31 / 1.29, of 700,001 (20 M) 7.7 / 5.9 /
 // 5.3 / 4.9 / 4.9, and 64 BFS 0.21 / 0.22 / 0.24 / 0.26 / 0.26, 0.34 / 0.32 / 0.33 /
-// 0.35 / 0.35, 1.38 / 1.11 / 0.99 / 0.93 / 0.93.  On a sparse graph a
+// 0.35 / 0.35, 1.38 / 1.11 / 0.99 / 0.93 / 0.93.  Beside the two steps, 32 BC: of 1.0,
+// 1.2 and 1.6 Mi edges 0.86 / 0.79 / 0.90 / 0.99 / 0.99, 0.92 / 0.87 / 0.96 / 1.04 / 1.04
+// and 1.00 / 0.87 / 0.93 / 0.96 / 0.95; of 7.8 and 8.6 Mi 3.12 / 2.46 / 2.25 / 2.20 / 2.20
+// and 3.69 / 2.96 / 2.67 / 2.61 / 2.60 (64 BFS within 5 % across each step).  On a sparse graph a
 // round's work grows with the sources times the wavefront (about sqrt(V) on
 // a grid), and a large one fills more blocks: push-only multi-source BFS, 64
 // sources on the 4096^2 grid 1030 / 650 / 521 / 462 ms with 1 / 2 / 3 / 4

@@ -76,3 +76,18 @@ def test_cpu_baseline_record():
     srcs = [int(s) for s in h.pick_sources(3, 3)]
     b = bench.cpu_baseline(h, srcs, budget_s=5.0)
     assert b["value"] > 0 and b["cores"] == 1 and b["kind"] in ("reference", "port") and b["unit"] == bench.METRIC
+
+
+def test_result_line_stays_short_beside_its_details():
+    import json
+
+    extra = {f"section{k}": {**{f"row{j}": {"x": 1.0, "parity": j != 3} for j in range(200)}, "bench_seconds": 2.0}
+             for k in range(4)}
+    line = {"metric": "GTEPS", "value": 1.0, "tuning": {"mode": "m", "autotune_report": ["r" * 100] * 100},
+            "parity": {"sssp": True}, "extra": extra}
+    short, details = bench.split_details(line)
+    assert len(json.dumps(short)) < 1500 and short["value"] == 1.0 and short["parity"]["sssp"]
+    assert details["extra"] == extra and len(details["autotune_report"]) == 100
+    assert len(details["parity"]) == short["parity"]["extra_checks"] == 800
+    assert len(short["parity"]["extra_failed"]) == 4
+    assert "autotune_report" in line["tuning"] and "extra" in line  # the argument is left as it was
