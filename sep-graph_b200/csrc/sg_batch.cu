@@ -949,8 +949,9 @@ sg_status prepare_batch(sg_ctx *ctx, sgb::Workspace &ws, std::vector<engine::Bat
     B.value_bytes = sizeof(TV);
     // unweighted batches take three blocks per SM when every graph is sparse (see
     // few_blocks), four otherwise: 32 BFS on the 512^2 grid 25.1 ms with three,
-    // 26.1 with four; on symmetric RMAT-18, pushing, 2.72 and 2.28
-    bool sparse = true;
+    // 26.1 with four; on symmetric RMAT-18, pushing, 2.72 and 2.28.  Contexts that
+    // share the device keep the four: half of three blocks is one.
+    bool sparse = ctx->resident_share == 1;
     for (auto *g : graphs) sparse = sparse && (double)g->ne < kFewBlocksDegree * g->nv;
     // per template instantiation: all variants, push, all variants for few blocks
     static std::atomic<int> occupancy[3] = {{0}, {0}, {0}};
